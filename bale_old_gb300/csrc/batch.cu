@@ -22,7 +22,7 @@
 // Instances large enough to fill the GPU by themselves (the standalone rule:
 // the partition thresholds, batch.standalone_min elements, or
 // batch.standalone_min_edges nonzeros for a graph) run their specialised
-// kernels instead -- region-partitioned ig / histo, the wedge triangle
+// kernels instead -- region-partitioned ig, bucketed histo, the wedge triangle
 // kernels -- on up to batch.streams captured side streams, longest first to
 // the least loaded, in parallel with the queue.  The whole run -- queue
 // reset, the persistent kernel and those launches -- is one CUDA graph,
@@ -341,11 +341,15 @@ void destroy(bale_batch *b) {
 }  // namespace
 namespace q {
 
-// Would this instance use the region-partitioned kernels on its own?
+// Would this instance use the bucketed or region-partitioned kernels on its
+// own?  The planner gives it a workspace for them.
+static bool bucketed(const bale_instance_t &x) {
+  return x.kind == BALE_KIND_HISTO && histo_mode_for(x.n, x.m, x.in, false) == 4;
+}
+
 bool partition_worthy(const bale_instance_t &x) {
   if (x.kind == BALE_KIND_IG) return ig_partition_for(x.n, x.m, x.out, x.in);
-  if (x.kind == BALE_KIND_HISTO) return histo_mode_for(x.n, x.m, x.in) == 3;
-  return false;
+  return x.kind == BALE_KIND_HISTO && histo_mode_for(x.n, x.m, x.in, false) >= 3;
 }
 
 // Instances large enough to fill the GPU by themselves run as their own
@@ -361,6 +365,7 @@ bool goes_standalone(const bale_instance_t &x) {
 size_t standalone_ws(const bale_instance_t &x) {
   size_t need = 0;
   if (x.kind == BALE_KIND_IG && partition_worthy(x)) need = ig_part_workspace_bytes(x.n, x.m);
+  else if (bucketed(x)) need = bucket_workspace_bytes(x.n, x.m);
   else if (x.kind == BALE_KIND_HISTO && partition_worthy(x)) need = histo_part_workspace_bytes(x.n, x.m);
   else if (x.kind == BALE_KIND_TRIANGLES)
     need = tri_wedge_supported(x.n, x.m) ? tri_wedge_workspace_bytes(x.n, x.m) : tri_hybrid_workspace_bytes(x.n, x.m);
@@ -379,8 +384,9 @@ int launch_standalone(const bale_instance_t &x, unsigned long long *bad, void *w
     return launch_ig(x.out, x.in, x.n, x.aux, x.m, x.shift, bad, st);
   }
   if (x.kind == BALE_KIND_HISTO) {
+    if (bucketed(x)) return launch_histo_bucket(x.out, x.m, x.in, x.n, x.shift, bad, ws, st);
     if (partition_worthy(x)) return launch_histo_partitioned(x.out, x.m, x.in, x.n, x.shift, bad, ws, words, st);
-    return launch_histo(x.out, x.m, x.in, x.n, x.shift, bad, st);
+    return launch_histo(x.out, x.m, x.in, x.n, x.shift, bad, st, false);
   }
   if (tri_wedge_supported(x.n, x.m))
     return launch_triangle_wedge(x.in, x.aux, x.n, x.m, reinterpret_cast<unsigned long long *>(x.out), nullptr, bad,

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
 #include "bale_gb300.h"
 
 namespace bale {
@@ -25,6 +27,8 @@ int64_t knob_or(const char *name, int64_t dflt);
 // enough elements to amortise the passes); thresholds are tuning knobs.
 bool ig_auto_partition(int64_t n, int64_t table_len);
 bool histo_auto_partition(int64_t n, int64_t ncounts);
+// ... and of the histogram by shared-memory buckets.
+bool histo_auto_bucket(int64_t n, int64_t ncounts);
 
 // Device-wide scratch words owned by the library (per device): the in-kernel
 // bad-input counter and the triangle work cursor.  Allocated once.
@@ -43,11 +47,23 @@ unsigned long long *next_cursor_words(int k);
 // different streams get their own.  Growing it frees the old buffer, which
 // waits for the device.  Returns nullptr (error set) on allocation failure.
 void *device_workspace(size_t bytes, cudaStream_t stream);
+// The bucketed gather's and histogram's workspaces, apart from the one above:
+// those calls used to need none, so they must not disturb, or be disturbed
+// by, another thread's launches on the same stream.  *hold keeps the pool
+// locked until the caller has enqueued all of its kernels.  At most
+// kBucketStreams streams keep one; the least recently used one goes first
+// (freeing it waits for the device).  Returns nullptr, with no error set,
+// when there is no memory: the caller then takes a path without one.
+constexpr int kBucketStreams = 8;
+void *bucket_workspace(size_t bytes, cudaStream_t stream, std::unique_lock<std::mutex> *hold);
+// Is work on this stream being captured into a graph?
+bool stream_capturing(cudaStream_t stream);
 // The launchers' choices, shared with the batched and serving planners so a
 // planner that supplies its own workspace takes the same path:
-// launch_histo's mode (0 shared memory, 1 aggregated, 2 plain, 3 partitioned)
-// and whether launch_ig uses the region partition.
-int histo_mode_for(int64_t n, int64_t ncounts, const int64_t *index);
+// launch_histo's mode (0 shared memory, 1 aggregated, 2 plain, 3 region
+// partition, 4 buckets) and launch_ig's path.  own_ws false: the buckets only
+// where the region partition would be taken, whose workspace is no smaller.
+int histo_mode_for(int64_t n, int64_t ncounts, const int64_t *index, bool own_ws = true);
 bool ig_partition_for(int64_t n, int64_t table_len, const int64_t *tgt, const int64_t *index);
 
 #define BALE_CUDA_OK(expr)                                                        \
@@ -61,10 +77,12 @@ bool ig_partition_for(int64_t n, int64_t table_len, const int64_t *tgt, const in
   } while (0)
 
 // Launch entry points used by the C ABI (all asynchronous on `stream`).
+// own_ws false: no workspace beyond the plan's own is taken for the bucketed
+// paths (the batch and serving planners account for memory themselves).
 int launch_ig(int64_t *tgt, const int64_t *index, int64_t n, const int64_t *table,
               int64_t table_len, int shift, unsigned long long *bad, cudaStream_t stream);
 int launch_histo(int64_t *counts, int64_t ncounts, const int64_t *index, int64_t n, int shift,
-                 unsigned long long *bad, cudaStream_t stream);
+                 unsigned long long *bad, cudaStream_t stream, bool own_ws = true);
 int launch_triangle(const int64_t *offset, const int64_t *nonzero, int64_t numrows, int64_t nnz,
                     unsigned long long *count, unsigned long long *work,
                     unsigned long long *bad, cudaStream_t stream);
@@ -91,6 +109,11 @@ size_t histo_part_workspace_bytes(int64_t n, int64_t ncounts);
 int launch_histo_partitioned(int64_t *counts, int64_t ncounts, const int64_t *index, int64_t n, int shift,
                              unsigned long long *bad, void *ws, unsigned long long *cursor,
                              cudaStream_t stream);
+// Histogram by shared-memory buckets of the table (bucket.cu).
+bool bucket_supported(int64_t n, int64_t ncounts);
+size_t bucket_workspace_bytes(int64_t n, int64_t ncounts);
+int launch_histo_bucket(int64_t *counts, int64_t ncounts, const int64_t *index, int64_t n, int shift,
+                        unsigned long long *bad, void *ws, cudaStream_t stream);
 // Bitmap/search hybrid triangle counting (tri_hybrid.cu); needs numrows < 2^32.
 size_t tri_hybrid_workspace_bytes(int64_t numrows, int64_t nnz);
 // run_if (optional, here and in the wedge functions below): a device word;

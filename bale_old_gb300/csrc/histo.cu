@@ -13,9 +13,12 @@
 //    (red.global.add.u64).  For tables that live in L2 this is bound by the
 //    L2 reduction rate, otherwise by one DRAM sector read and write-back per
 //    update;
-//  * tables well beyond L2: the updates are first partitioned by 16 MiB
-//    region (ig_part.cu's partition), so the reductions of one region at a
-//    time stay in L2;
+//  * larger tables with millions of updates: the updates are first sorted
+//    into slices of the table that fit shared memory, and counted there
+//    (histo_bucket.cu);
+//  * tables beyond that one's range (75 M counters): the updates are first
+//    partitioned by 16 MiB region (ig_part.cu's partition), so the reductions
+//    of one region at a time stay in L2;
 //  * skewed updates (mode 1, chosen by the tuner or the caller): the lanes
 //    that hit the same counter are grouped with __match_any_sync and the
 //    leader adds the group size with one reduction.
@@ -164,32 +167,46 @@ int launch_l2_red_rate(int64_t *counts, int64_t ncounts, int64_t n, cudaStream_t
 }
 
 // Mode: 0 shared-memory private table, 1 warp-aggregated L2 reductions,
-// 2 plain L2 reductions, 3 region-partitioned L2 reductions.  Automatic:
-// shared memory when the table fits; plain L2 reductions while the table
-// lives in L2 (uniform updates rarely collide inside a warp, so the
-// aggregation's __match_any_sync costs more than it saves -- it pays only
-// for skewed updates, which the tuner or the caller can select); the
-// region partition once the table is well beyond L2.
-int histo_mode_for(int64_t n, int64_t ncounts, const int64_t *index) {
+// 2 plain L2 reductions, 3 region-partitioned L2 reductions, 4 shared-memory
+// buckets.  Automatic: shared memory when the table fits; with enough updates
+// the shared-memory buckets, and beyond their range the region partition;
+// plain L2 reductions otherwise (uniform updates rarely collide inside a
+// warp, so the aggregation's __match_any_sync costs more than it saves: 10^7
+// updates of 10^6 counters 151 us against 55, and 233 against 608 for
+// Zipf(1.1), which the tuner or the caller can select it for).  The buckets
+// need a workspace of 2 bytes per update; where that cannot be had, or the
+// stream is being captured and the call did not need one before, it takes the
+// path it would take without them.
+int histo_mode_for(int64_t n, int64_t ncounts, const int64_t *index, bool own_ws) {
   const bool aligned = (reinterpret_cast<uintptr_t>(index) & 15) == 0;
   int64_t mode = knob("histo.mode");
-  if (mode < 0 || mode > 3) {
+  if (mode < 0 || mode > 4) {
+    const bool part = histo_auto_partition(n, ncounts);
     if (ncounts <= kSmemMaxCounters) mode = 0;
-    else if (histo_auto_partition(n, ncounts)) mode = 3;
+    else if (bucket_supported(n, ncounts) && (part || (own_ws && histo_auto_bucket(n, ncounts)))) mode = 4;
+    else if (part) mode = 3;
     else mode = 2;
   }
   if (mode == 0 && ncounts > kSmemMaxCounters) mode = 2;
-  if (!aligned && (mode == 0 || mode == 3)) mode = 2;
+  if (mode == 4 && !bucket_supported(n, ncounts)) mode = 2;
+  if (!aligned && mode != 1) mode = 2;
   if (mode == 3 && ncounts > (kIgMaxRegions << kIgRegionBits)) mode = 2;
   return static_cast<int>(mode);
 }
 
 int launch_histo(int64_t *counts, int64_t ncounts, const int64_t *index, int64_t n, int shift,
-                 unsigned long long *bad, cudaStream_t stream) {
+                 unsigned long long *bad, cudaStream_t stream, bool own_ws) {
   if (n <= 0) return BALE_OK;
   const int sms = num_sms();
   const bool aligned = (reinterpret_cast<uintptr_t>(index) & 15) == 0;
-  const int64_t mode = histo_mode_for(n, ncounts, index);
+  int64_t mode = histo_mode_for(n, ncounts, index, own_ws);
+  if (mode == 4 && own_ws && stream_capturing(stream)) mode = histo_mode_for(n, ncounts, index, false);
+  if (mode == 4) {
+    std::unique_lock<std::mutex> hold;
+    void *ws = bucket_workspace(bucket_workspace_bytes(n, ncounts), stream, &hold);
+    if (ws) return launch_histo_bucket(counts, ncounts, index, n, shift, bad, ws, stream);
+    mode = histo_auto_partition(n, ncounts) ? 3 : 2;
+  }
   if (mode == 3) {
     void *ws = device_workspace(histo_part_workspace_bytes(n, ncounts), stream);
     unsigned long long *cursor = next_cursor_word();

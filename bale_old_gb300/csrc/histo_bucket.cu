@@ -1,0 +1,427 @@
+// histo_bucket.cu -- histogram by shared-memory buckets of the counters, for
+// tables too large for one CTA's shared memory.
+//
+// A reduction at L2 runs at 178 G/s at best, at 60 G/s once the counters
+// outgrow L2, and at a few G/s per address when the updates are skewed.
+// Shared memory takes several times that, so the counters are cut into slices
+// ("buckets") that fit it -- bale's exstack (apps/histo_src/
+// histo_exstack.upc:64-76) with the buckets in the place of the PEs:
+//
+//  1. partition: each chunk of 12288 updates is counting-sorted by bucket in
+//     shared memory and written back as 16-bit offsets inside the bucket,
+//     with the chunk's bucket boundaries;
+//  2. count: per bucket, a CTA walks the chunks' segments of that bucket,
+//     counts in shared memory and adds its counts to the table with coalesced
+//     reductions (the table stays safe against concurrent calls).
+//
+// The streams are 8 + 2 + 2 bytes per update, and 16 per counter and part.
+// Measured (us, before: plain L2 reductions, or the region partition for 2^26
+// updates of 2^24 counters; after): 10^7 updates of 10^6 counters 54.5 -> 48
+// (partition 26, count 21), 2^26 of 2^24 counters 553 -> 299 (partition 137,
+// count 140), 2^26 of 10^6 373 -> 181; Zipf(1.1) 2^26 of 2^24 counters 6230 ->
+// 290.  The partition is bound by its shared-memory accesses (77% of the
+// LSU data pipe) and reads at 4.9 TB/s; the count by the latency of its short
+// segments (13 entries at 2^24 counters).
+//
+// Skewed updates fill some buckets far more than others, so a bucket is cut
+// into parts (ranges of chunks) by its share of a sample of the chunks, which
+// the partition counts; each part is an item that one CTA walks.
+#include <algorithm>
+
+#include "common.cuh"
+
+namespace bale {
+
+namespace {
+
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kPartThreads = 512;
+constexpr int kPer = 24;                     // updates per thread of the partition
+constexpr int kChunk = kPartThreads * kPer;  // 12288 updates per chunk
+constexpr int kPartBlocks = 3;               // per SM
+constexpr int kCountThreads = 512;
+constexpr int kCountBlocks = 3;              // per SM
+constexpr uint32_t kBucket = 18432;          // at most this many counters per bucket: 72 KiB of u32
+constexpr uint32_t kMinBucket = 8192;
+constexpr int kMaxBuckets = 4094;
+constexpr int kSampleEvery = 4;              // chunks per chunk counted for the parts
+// Workspace words: the next item, and each bucket's updates in the sampled chunks.
+constexpr int kWordNext = 0, kWordTotals = 32;
+
+// Bucket of table entry k: k / size, by a multiplication that is exact for
+// k < 2^30 and 2^13 <= size < 2^15 (magic = ceil(2^45 / size) exceeds
+// 2^45 / size by less than 1, so k * magic is off by less than 2^45 / size).
+struct Buckets {
+  uint32_t size, magic;
+  int n;
+};
+__device__ __forceinline__ uint32_t bucket_of(uint32_t k, Buckets bk) { return __umulhi(k, bk.magic) >> 13; }
+
+static_assert(kChunk <= 65536, "positions and boundaries are 16 bits");
+static_assert(kPer % 8 == 0 && kChunk % 8 == 0, "whole 16-byte vectors");
+
+// Boundaries: 8 chunks' values of one bucket side by side, so the partition's
+// stores and the walk's loads both touch few lines.
+__device__ __forceinline__ size_t start_at(int64_t c, int b, int nbp) {
+  return ((static_cast<size_t>(c >> 3) * nbp + b) << 3) | static_cast<size_t>(c & 7);
+}
+
+__device__ __forceinline__ uint32_t incl_scan_u32(uint32_t v) {
+  const unsigned lane = lane_id();
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, v, o);
+    if (static_cast<int>(lane) >= o) v += y;
+  }
+  return v;
+}
+
+// A predicated reduction, written out, because the compiler branches around a
+// conditional shared-memory reduction (29 instructions per reduction, where
+// the predicated form needs 4).
+__device__ __forceinline__ void red_shared_if(uint32_t pred, uint32_t addr) {
+  asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p red.shared.add.u32 [%1], 1; }" ::"r"(pred), "r"(addr)
+               : "memory");
+}
+
+// Exclusive scan of a[0,m) in shared memory, in place, by the whole block;
+// a[m] = the total.
+__device__ __forceinline__ void block_scan(uint32_t *a, int m, uint32_t *warp_tot) {
+  const int per = (m + kPartThreads - 1) / kPartThreads;
+  const int lo = threadIdx.x * per, hi = min(lo + per, m);
+  uint32_t sum = 0;
+  for (int i = lo; i < hi; i++) sum += a[i];
+  const uint32_t inc = incl_scan_u32(sum);
+  if (lane_id() == 31) warp_tot[threadIdx.x >> 5] = inc;
+  __syncthreads();
+  uint32_t run = inc - sum;
+  for (unsigned w = 0; w < (threadIdx.x >> 5); w++) run += warp_tot[w];
+  for (int i = lo; i < hi; i++) {
+    const uint32_t v = a[i];
+    a[i] = run;
+    run += v;
+  }
+  if (threadIdx.x == kPartThreads - 1) a[m] = run;
+  __syncthreads();
+}
+
+template <int SHIFT, bool WHOLE>
+__device__ __forceinline__ void partition_chunk(const int64_t *__restrict__ index, int64_t n, uint64_t ncounts,
+                                                Buckets bk, uint16_t *__restrict__ off16,
+                                                uint16_t *__restrict__ starts, uint32_t *__restrict__ words,
+                                                unsigned long long *__restrict__ bad, uint32_t *hist, uint16_t *stage,
+                                                uint32_t *warp_tot) {
+  const int t = threadIdx.x, nb = bk.n;
+  const int64_t c = blockIdx.x, base = c * kChunk;
+  const int len = WHOLE ? kChunk : static_cast<int>(n - base);
+  const uint64_t pol = policy_evict_first();
+  for (int i = t; i < nb + 2; i += kPartThreads) hist[i] = 0;
+  __syncthreads();
+  uint32_t key[kPer];  // bucket << 16 | offset in the bucket; bucket nb for an out-of-range update
+  const longlong2 *src = reinterpret_cast<const longlong2 *>(index + base);
+#pragma unroll
+  for (int h = 0; h < kPer / 2; h++) {
+    longlong2 v;
+    const int e0 = 2 * (h * kPartThreads + t);  // position in the chunk of v.x
+    if (WHOLE) {
+      v = ld_v2_s64_pol(src + h * kPartThreads + t, pol);
+    } else {
+      v.x = e0 < len ? index[base + e0] : 0;
+      v.y = e0 + 1 < len ? index[base + e0 + 1] : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const uint64_t k = static_cast<uint64_t>((j ? v.y : v.x) >> SHIFT);
+      const uint32_t k32 = static_cast<uint32_t>(k), b = bucket_of(k32, bk);
+      const uint32_t kk = k < ncounts ? (b << 16 | (k32 - b * bk.size)) : static_cast<uint32_t>(nb) << 16;
+      key[2 * h + j] = kk;
+      if (WHOLE || e0 + j < len) atomicAdd(&hist[kk >> 16], 1u);
+    }
+  }
+  __syncthreads();
+  block_scan(hist, nb + 1, warp_tot);
+  const bool counted = c % kSampleEvery == 0;
+  for (int i = t; i < nb + 2; i += kPartThreads) {
+    const uint32_t at = hist[i];
+    starts[start_at(c, i, nb + 2)] = static_cast<uint16_t>(at);
+    if (counted && i < nb) atomicAdd(words + kWordTotals + i, hist[i + 1] - at);
+  }
+  if (t == 0 && hist[nb + 1] != hist[nb]) atomicAdd(bad, static_cast<unsigned long long>(hist[nb + 1] - hist[nb]));
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < kPer; s++)
+    if (WHOLE || 2 * ((s >> 1) * kPartThreads + t) + (s & 1) < len)
+      stage[atomicAdd(&hist[key[s] >> 16], 1u)] = static_cast<uint16_t>(key[s]);
+  __syncthreads();
+  // a partial chunk's last vector carries unused entries (off16 holds whole chunks)
+  uint4 *o = reinterpret_cast<uint4 *>(off16 + base);
+  for (int i = t; i < (len + 7) / 8; i += kPartThreads) o[i] = reinterpret_cast<const uint4 *>(stage)[i];
+}
+
+template <int SHIFT>
+__global__ void __launch_bounds__(kPartThreads, kPartBlocks)
+    bucket_partition_kernel(const int64_t *__restrict__ index, int64_t n, uint64_t ncounts, Buckets bk,
+                            uint16_t *__restrict__ off16, uint16_t *__restrict__ starts, uint32_t *__restrict__ words,
+                            unsigned long long *__restrict__ bad) {
+  extern __shared__ __align__(16) uint16_t stage[];  // kChunk entries, then nb + 2 counts
+  __shared__ uint32_t warp_tot[kPartThreads / 32];
+  uint32_t *hist = reinterpret_cast<uint32_t *>(stage + kChunk);
+  if ((static_cast<int64_t>(blockIdx.x) + 1) * kChunk <= n)
+    partition_chunk<SHIFT, true>(index, n, ncounts, bk, off16, starts, words, bad, hist, stage, warp_tot);
+  else
+    partition_chunk<SHIFT, false>(index, n, ncounts, bk, off16, starts, words, bad, hist, stage, warp_tot);
+}
+
+// The items: bucket b is cut into parts(b) = its sampled requests * scale,
+// rounded up, at least one.  ends[b] = the parts of buckets 0..b, below 2^16
+// because the parts beyond one per bucket are at most a few per CTA; called
+// by the whole block, which learns the number of items.
+template <int THREADS>
+__device__ __forceinline__ uint32_t plan_items(const uint32_t *__restrict__ words, int nb, float scale,
+                                               uint32_t nchunks, uint16_t *ends, uint32_t *warp_tot) {
+  const int per = (nb + THREADS - 1) / THREADS, lo = threadIdx.x * per, hi = min(lo + per, nb);
+  uint32_t sum = 0;
+  for (int b = lo; b < hi; b++) {
+    const uint32_t parts = static_cast<uint32_t>(ceilf(static_cast<float>(words[kWordTotals + b]) * scale));
+    sum += min(max(parts, 1u), nchunks);
+    ends[b] = static_cast<uint16_t>(sum);
+  }
+  const uint32_t inc = incl_scan_u32(sum);
+  if (lane_id() == 31) warp_tot[threadIdx.x >> 5] = inc;
+  __syncthreads();
+  uint32_t before = inc - sum;
+  for (unsigned w = 0; w < (threadIdx.x >> 5); w++) before += warp_tot[w];
+  for (int b = lo; b < hi; b++) ends[b] = static_cast<uint16_t>(ends[b] + before);
+  __syncthreads();
+  return ends[nb - 1];
+}
+
+// A block's item: bucket b, chunks [c0, c1).
+struct Item {
+  int b;
+  uint32_t c0, c1;
+};
+
+__device__ __forceinline__ Item find_item(uint32_t it, const uint16_t *ends, int nb, uint32_t nchunks) {
+  int lo = 0, hi = nb - 1;
+  while (lo < hi) {  // the first bucket with ends > it
+    const int mid = (lo + hi) >> 1;
+    if (ends[mid] > it) hi = mid; else lo = mid + 1;
+  }
+  const uint32_t first = lo ? ends[lo - 1] : 0u, parts = ends[lo] - first, p = it - first;
+  return {lo, static_cast<uint32_t>(static_cast<uint64_t>(nchunks) * p / parts),
+          static_cast<uint32_t>(static_cast<uint64_t>(nchunks) * (p + 1) / parts)};
+}
+
+// A warp's share of an item: groups of up to 32 chunks, every WARPS-th, cut so
+// that all warps get the same number.  The boundaries of a group are loaded
+// one group ahead of its walk.
+//
+// A segment holds a dozen or a few hundred entries, and every step to the next
+// one is a dependent access of a microsecond, so nothing here waits on a
+// global atomic: with the chunks claimed from a cursor per bucket, 40% of the
+// time went into the claims that open a bucket (2^26 updates of 2^24
+// counters: 207 us for this kernel, against 139).
+template <int WARPS>
+struct Groups {
+  const uint16_t *__restrict__ starts;  // of bucket b
+  uint32_t pitch, at, step, size, end;
+  uint32_t se;  // this lane's segment of the group at `at`: start | end << 16
+
+  __device__ __forceinline__ uint32_t boundaries(uint32_t c) const {
+    const uint16_t *st = starts + static_cast<uint64_t>(c >> 3) * pitch + (c & 7u);
+    return static_cast<uint32_t>(st[0]) | static_cast<uint32_t>(st[8]) << 16;
+  }
+  __device__ __forceinline__ void load() {
+    const uint32_t c = at + lane_id();
+    se = lane_id() < size && c < end ? boundaries(c) : 0u;
+  }
+  __device__ __forceinline__ void begin(const uint16_t *all_starts, int nb, Item it) {
+    starts = all_starts + static_cast<size_t>(it.b) * 8;
+    pitch = static_cast<uint32_t>(nb + 2) * 8u;
+    const uint32_t range = it.c1 - it.c0, k = (range + WARPS * 32 - 1) / (WARPS * 32);
+    size = k ? (range + WARPS * k - 1) / (WARPS * k) : 1u;
+    step = size * WARPS;
+    at = it.c0 + size * (threadIdx.x >> 5);
+    end = it.c1;
+    load();
+  }
+  // f(c, mine) for every group: its first chunk, this lane's segment.
+  template <class F>
+  __device__ __forceinline__ void run(F f) {
+    while (at < end) {
+      const uint32_t c = at, mine = se;
+      at += step;
+      load();
+      f(c, mine);
+    }
+  }
+};
+
+// One group of the histogram: cnts[ent[i]]++ for every entry i, eight
+// entries per 16-byte load.  The segments' vectors are flattened over the
+// lanes: the owner of a flattened place is found from the segments' first
+// places, one bit each in a window of 32 (an OR over the warp).
+__device__ __forceinline__ void count_vec(uint32_t cnts, uint4 x, uint32_t mask) {
+  const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    red_shared_if(mask & (1u << k), cnts + 4u * (k & 1 ? w[k >> 1] >> 16 : w[k >> 1] & 0xffffu));
+}
+
+__device__ __forceinline__ void count_group(const uint4 *__restrict__ ent, uint32_t cnts, uint32_t mine) {
+  constexpr int kVecs = 3;  // vectors in flight per lane
+  constexpr uint32_t kChunkVecs = kChunk / 8;
+  const unsigned lane = lane_id();
+  const uint32_t le = (2u << lane) - 1u;
+  const uint32_t s = mine & 0xffffu, e = mine >> 16, v0 = s >> 3, nv = e > s ? ((e + 7u) >> 3) - v0 : 0u;
+  const uint32_t inc = incl_scan_u32(nv), tot = __shfl_sync(kFull, inc, 31);
+  const uint32_t ex = nv ? inc - nv : 0xffffff00u;         // beyond any window
+  const uint32_t rel = lane * kChunkVecs + v0 - (inc - nv);  // vector index - flattened place
+  uint32_t before = 0;  // segments that begin before the window
+  // lanes with vectors, in order: the segment with k others before it
+  const unsigned live = __ballot_sync(kFull, nv > 0);
+  const bool packed = (live & (live + 1u)) == 0;  // nearly always
+  for (uint32_t bb = 0; bb < tot; bb += 32 * kVecs) {
+    uint4 x[kVecs];
+    uint32_t mask[kVecs];
+#pragma unroll
+    for (int u = 0; u < kVecs; u++) {
+      const uint32_t at = bb + 32u * u, d = ex - at;
+      const uint32_t win = __reduce_or_sync(kFull, d < 32u ? 1u << d : 0u);
+      const uint32_t o = before + __popc(win & le) - 1u;
+      before += __popc(win);
+      const int src = packed ? static_cast<int>(o) : static_cast<int>(__fns(live, 0, static_cast<int>(o) + 1));
+      const uint32_t q = __shfl_sync(kFull, rel, src) + at + lane;
+      const uint32_t se = __shfl_sync(kFull, mine, src);
+      const uint32_t i0 = (q - static_cast<uint32_t>(src) * kChunkVecs) * 8u;  // the vector's first entry in its chunk
+      const int lo = static_cast<int>(se & 0xffffu) - static_cast<int>(i0), hi = static_cast<int>(se >> 16) - static_cast<int>(i0);
+      const bool in = at + lane < tot;
+      mask[u] = in ? (0xffu >> max(0, 8 - hi)) & (0xffu << max(0, lo)) : 0u;
+      x[u] = in ? __ldg(ent + q) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < kVecs; u++) count_vec(cnts, x[u], mask[u]);
+  }
+}
+
+__global__ void __launch_bounds__(kCountThreads, kCountBlocks)
+    bucket_count_kernel(const uint16_t *__restrict__ off16, const uint16_t *__restrict__ starts, int64_t nchunks,
+                        Buckets bk, float scale, int64_t *__restrict__ counts, uint64_t ncounts,
+                        uint32_t *__restrict__ words) {
+  extern __shared__ __align__(16) uint32_t cnts[];  // bk.size counters rounded up to 4, then the item plan
+  __shared__ uint32_t warp_tot[kCountThreads / 32], post[2];
+  const uint32_t cnts_at = static_cast<uint32_t>(__cvta_generic_to_shared(cnts));
+  const uint32_t nch = static_cast<uint32_t>(nchunks), quads = (bk.size + 3u) / 4u;
+  uint16_t *ends = reinterpret_cast<uint16_t *>(cnts + quads * 4u);
+  const uint32_t items = plan_items<kCountThreads>(words, bk.n, scale, nch, ends, warp_tot);
+  Groups<kCountThreads / 32> gr;
+  uint32_t it = blockIdx.x;
+  Item x = {0, 0, 0};
+  if (it < items) {
+    x = find_item(it, ends, bk.n, nch);
+    gr.begin(starts, bk.n, x);
+  }
+  for (int turn = 0; it < items; turn ^= 1) {
+    uint32_t asked = 0;
+    if (threadIdx.x == 0) asked = gridDim.x + atomicAdd(words + kWordNext, 1u);
+    for (uint32_t i = threadIdx.x; i < quads; i += kCountThreads) reinterpret_cast<uint4 *>(cnts)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x == 0) post[turn] = asked;
+    __syncthreads();
+    gr.run([&](uint32_t c, uint32_t mine) {
+      count_group(reinterpret_cast<const uint4 *>(off16 + static_cast<int64_t>(c) * kChunk), cnts_at, mine);
+    });
+    __syncthreads();
+    // the next item's first boundaries load while this one's counters leave
+    const Item done = x;
+    it = post[turn];
+    if (it < items) {
+      x = find_item(it, ends, bk.n, nch);
+      gr.begin(starts, bk.n, x);
+    }
+    const uint64_t t0 = static_cast<uint64_t>(done.b) * bk.size;
+    const uint32_t have = static_cast<uint32_t>(min(static_cast<uint64_t>(bk.size), ncounts - t0));
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < have; i += kCountThreads) {
+      const uint32_t v = cnts[i];
+      if (v) red_add_u64(counts + t0 + i, v);
+    }
+    __syncthreads();
+  }
+}
+
+size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
+
+// The buckets of a table of ncounts counters for `slots` CTAs: as large as
+// allowed, their number then raised to fill whole rounds of the CTAs (or, for
+// fewer buckets than CTAs, so that whole parts of each do).
+Buckets choose_buckets(int64_t ncounts, int64_t slots) {
+  int64_t nb = (ncounts + kBucket - 1) / kBucket;
+  if (nb >= slots) nb = std::min<int64_t>((nb + slots - 1) / slots * slots, std::max<int64_t>(nb, kMaxBuckets));
+  else nb = slots / (slots / nb);
+  Buckets bk;
+  bk.size = static_cast<uint32_t>(std::max<int64_t>(kMinBucket, (ncounts + nb - 1) / nb));
+  bk.n = static_cast<int>((ncounts + bk.size - 1) / bk.size);
+  bk.magic = static_cast<uint32_t>(((uint64_t(1) << 45) + bk.size - 1) / bk.size);
+  return bk;
+}
+
+// Parts per sampled request: an even share of the work per CTA, with a margin
+// so that evenly filled buckets are cut alike.
+float part_scale(int64_t n, const Buckets &bk, int64_t slots) {
+  const int64_t each = std::max<int64_t>(1, slots / bk.n);
+  return static_cast<float>(kSampleEvery * static_cast<double>(bk.n) * each / (static_cast<double>(n) * (each > 1 ? 1.05 : 1.5)));
+}
+
+int64_t walk_slots() { return static_cast<int64_t>(num_sms()) * kCountBlocks; }
+
+// Workspace: words, boundaries, offsets.
+struct Layout {
+  int64_t nchunks;
+  Buckets bk;
+  size_t words_bytes, starts, off16, total;
+};
+
+Layout layout(int64_t n, int64_t ncounts) {
+  Layout l;
+  l.nchunks = (n + kChunk - 1) / kChunk;
+  l.bk = choose_buckets(ncounts, walk_slots());
+  l.words_bytes = (kWordTotals + static_cast<size_t>(l.bk.n)) * 4;
+  l.starts = up256(l.words_bytes);
+  l.off16 = l.starts + up256(static_cast<size_t>((l.nchunks + 7) / 8) * 8 * (l.bk.n + 2) * 2);
+  l.total = l.off16 + up256(static_cast<size_t>(l.nchunks) * kChunk * 2);
+  return l;
+}
+
+}  // namespace
+
+bool bucket_supported(int64_t n, int64_t ncounts) {
+  // n: an item's updates fit a u32 counter however skewed they are
+  return n > 0 && n < (int64_t(1) << 32) && ncounts > 0 && ncounts <= static_cast<int64_t>(kMaxBuckets) * kBucket;
+}
+
+size_t bucket_workspace_bytes(int64_t n, int64_t ncounts) { return layout(n, ncounts).total; }
+
+int launch_histo_bucket(int64_t *counts, int64_t ncounts, const int64_t *index, int64_t n, int shift,
+                        unsigned long long *bad, void *ws, cudaStream_t stream) {
+  const Layout l = layout(n, ncounts);
+  char *p = static_cast<char *>(ws);
+  uint32_t *words = reinterpret_cast<uint32_t *>(p);
+  uint16_t *starts = reinterpret_cast<uint16_t *>(p + l.starts), *off16 = reinterpret_cast<uint16_t *>(p + l.off16);
+  BALE_CUDA_OK(cudaMemsetAsync(words, 0, l.words_bytes, stream));
+  auto part = shift == 16 ? bucket_partition_kernel<16> : bucket_partition_kernel<0>;
+  const int psmem = kChunk * 2 + (l.bk.n + 2) * 4;
+  BALE_CUDA_OK(cudaFuncSetAttribute(part, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem));
+  part<<<static_cast<unsigned>(l.nchunks), kPartThreads, psmem, stream>>>(index, n, static_cast<uint64_t>(ncounts),
+                                                                         l.bk, off16, starts, words, bad);
+  BALE_CUDA_OK(cudaGetLastError());
+  const int csmem = static_cast<int>((l.bk.size + 3) / 4 * 16 + l.bk.n * 2);
+  BALE_CUDA_OK(cudaFuncSetAttribute(bucket_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, csmem));
+  const int64_t slots = walk_slots();
+  bucket_count_kernel<<<static_cast<unsigned>(slots), kCountThreads, csmem, stream>>>(
+      off16, starts, l.nchunks, l.bk, part_scale(n, l.bk, slots), counts, static_cast<uint64_t>(ncounts), words);
+  BALE_CUDA_OK(cudaGetLastError());
+  return BALE_OK;
+}
+
+}  // namespace bale

@@ -24,6 +24,8 @@
 // merge kernel), 1 (tri_hybrid.cu), 2 (tri_wedge.cu) and the default, whose
 // per-graph choice between wedges and the hybrid is made on the device
 // (tri_choose_kernel below).
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace bale {
@@ -198,11 +200,12 @@ __global__ void __launch_bounds__(kChooseThreads)
     const int64_t d = off[i + 1] - off[i];
     if (d > 1) pushes += static_cast<unsigned long long>(d) * static_cast<unsigned long long>(d - 1) / 2;
   }
-  if (blockIdx.x == 0 && nnz > 0) {
-    for (int s = threadIdx.x; s < kChooseSamples; s += kChooseThreads) {
-      const int64_t j = col[static_cast<int64_t>((static_cast<unsigned long long>(s) * nnz) / kChooseSamples)];
-      if (j >= 0 && j < n) pulls += static_cast<unsigned long long>(off[j + 1] - off[j]);  // a bad j: the paths count it
-    }
+  // a sample is two dependent loads, so the samples are spread over all
+  // threads (in one block they took 22 us)
+  for (int64_t s = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; nnz > 0 && s < kChooseSamples;
+       s += stride) {
+    const int64_t j = col[static_cast<int64_t>((static_cast<unsigned long long>(s) * nnz) / kChooseSamples)];
+    if (j >= 0 && j < n) pulls += static_cast<unsigned long long>(off[j + 1] - off[j]);  // a bad j: the paths count it
   }
   pushes = warp_sum_u64(pushes);
   pulls = warp_sum_u64(pulls);
@@ -232,11 +235,11 @@ int launch_triangle(const int64_t *offset, const int64_t *nonzero, int64_t numro
   // this file's warp-per-row merge kernel for every row.
   const int64_t mode = knob("tri.mode");
   if (mode < 0 && tri_wedge_supported(numrows, nnz) && nnz >= knob_or("tri.choose_min_nnz", kChooseMinNnz)) {
-    // both paths launched, the one not chosen returning at once; their
-    // workspaces side by side
-    const size_t wbytes = (tri_wedge_workspace_bytes(numrows, nnz) + 255) & ~size_t(255);
-    char *ws = static_cast<char *>(device_workspace(wbytes + tri_hybrid_workspace_bytes(numrows, nnz), stream));
-    unsigned long long *cursor = next_cursor_words(2), *hwords = next_cursor_words(3), *cw = next_cursor_words(4);
+    // both paths launched, the one not chosen returning at once, so they share
+    // one workspace
+    void *ws = device_workspace(
+        std::max(tri_wedge_workspace_bytes(numrows, nnz), tri_hybrid_workspace_bytes(numrows, nnz)), stream);
+    unsigned long long *cursor = next_cursor_words(2), *hwords = next_cursor_words(4), *cw = next_cursor_words(4);
     if (!ws || !cursor || !hwords || !cw) return BALE_ENOMEM;
     unsigned *choice = reinterpret_cast<unsigned *>(cw + 3);
     BALE_CUDA_OK(cudaMemsetAsync(cw, 0, 3 * sizeof(unsigned long long), stream));
@@ -251,7 +254,7 @@ int launch_triangle(const int64_t *offset, const int64_t *nonzero, int64_t numro
     if (rc != BALE_OK) return rc;
     int64_t rpf_h = knob("tri.rows_per_fetch");
     if (rpf_h < 1 || rpf_h > 4096) rpf_h = 8;
-    return launch_triangle_hybrid(offset, nonzero, numrows, nnz, count, work, bad, ws + wbytes, hwords,
+    return launch_triangle_hybrid(offset, nonzero, numrows, nnz, count, work, bad, ws, hwords,
                                   static_cast<int>(rpf_h), stream, choice);
   }
   if ((mode < 0 || mode == 2) && tri_wedge_supported(numrows, nnz)) {
@@ -264,7 +267,7 @@ int launch_triangle(const int64_t *offset, const int64_t *nonzero, int64_t numro
     int64_t rpf_h = knob("tri.rows_per_fetch");
     if (rpf_h < 1 || rpf_h > 4096) rpf_h = 8;
     void *ws = device_workspace(tri_hybrid_workspace_bytes(numrows, nnz), stream);
-    unsigned long long *words = next_cursor_words(3);
+    unsigned long long *words = next_cursor_words(4);
     if (!ws || !words) return BALE_ENOMEM;
     return launch_triangle_hybrid(offset, nonzero, numrows, nnz, count, work, bad, ws, words,
                                   static_cast<int>(rpf_h), stream);

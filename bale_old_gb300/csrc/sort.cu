@@ -2,8 +2,8 @@
 // scan the graph build and spmat's operations share.
 //
 // The radix sort takes 8 bits per pass over tiles of 4096 keys.  In a pass,
-// every key's rank among equal digits of its tile comes from a warp match and
-// per-warp counts in shared memory; the tile is laid out in shared memory in
+// every key's rank among equal digits of its tile comes from the lanes of its
+// warp with the same digit and per-warp counts in shared memory; the tile is laid out in shared memory in
 // sorted order and leaves run by run.  Where a tile's runs start in the
 // output comes, below 2^30 keys, from a single sweep (the published Onesweep
 // scheme of Adinets and Merrill, 2022): one histogram kernel counts the
@@ -130,6 +130,12 @@ __global__ void __launch_bounds__(kThreads)
 constexpr int kWarpSlice = static_cast<int>(kTile) / kWarps;  // 512 keys per warp
 static_assert(kWarpSlice == 32 * kPer, "a warp's slice is kPer rounds of 32");
 
+// Ranking rounds by a warp match: one in this many, the others by bits set in
+// shared memory.  Matches alone keep the ADU pipe at 75% and take 141 us for a
+// pass over 2^24 keys, bits alone the LSU data pipe at 78% and take 115; in
+// turn the two pipes share the work: 110.
+constexpr int kMatchEvery = 2;
+
 // A single-sweep pass's tile words: flag in the top two bits, a count below.
 constexpr uint32_t kStAggregate = 1u << 30;  // the tile's own digit count
 constexpr uint32_t kStPrefix = 2u << 30;     // the count of the digit in this and every earlier tile
@@ -207,14 +213,18 @@ template <bool LOOKBACK>
 __global__ void __launch_bounds__(kThreads, 4)
     radix_scatter_kernel(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int64_t n, int shift,
                          const uint32_t *__restrict__ offs, int64_t ntiles, Lookback lb) {
-  __shared__ uint64_t sorted[kTile];
-  __shared__ uint32_t wcnt[kWarps][kDigits];  // counts per warp, then their exclusive prefix over warps
+  __shared__ __align__(16) uint64_t sorted[kTile];
+  __shared__ uint32_t wcnt[kWarps][kDigits];  // exclusive prefix over warps of the digit counts
   __shared__ uint32_t gbase[kDigits];         // where each digit's run starts in dst
   __shared__ uint32_t wsum[kWarps];
   __shared__ uint32_t claimed;
   const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+  // until the layout, sorted's space holds each warp's digit words: the lanes
+  // with the digit in this round (x) and the digit's keys so far (y)
+  uint2(*words)[kDigits] = reinterpret_cast<uint2(*)[kDigits]>(sorted);
+  static_assert(sizeof(uint2) * kWarps * kDigits <= sizeof(sorted), "the words fit");
 #pragma unroll
-  for (int w = 0; w < kWarps; w++) wcnt[w][threadIdx.x] = 0;
+  for (int w = 0; w < kWarps; w++) words[w][threadIdx.x] = make_uint2(0u, 0u);
   if constexpr (LOOKBACK) {
     if (threadIdx.x == 0) claimed = atomicAdd(lb.counter, 1u);
     lb.next[static_cast<int64_t>(blockIdx.x) * kDigits + threadIdx.x] = 0;
@@ -228,19 +238,38 @@ __global__ void __launch_bounds__(kThreads, 4)
   uint64_t key[kPer];
   uint32_t dr[kPer];  // digit << 16 | rank among the warp's keys of that digit (kDigits: no key)
 #pragma unroll
+  for (int r = 0; r < kPer; r++) key[r] = first + r * 32 < n ? src[first + r * 32] : 0ull;
+#pragma unroll
   for (int r = 0; r < kPer; r++) {
-    const int64_t i = first + r * 32;
-    const bool valid = i < n;
-    key[r] = valid ? src[i] : 0ull;
-    const uint32_t d = valid ? static_cast<uint32_t>(key[r] >> shift) & (kDigits - 1) : kDigits;
-    // the lowest lane of each digit adds the digit's keys to the warp's count
-    // and hands the count before them to the others
-    const unsigned peers = __match_any_sync(kFull, d);
-    const uint32_t below = __popc(peers & ((1u << lane) - 1u));
-    uint32_t prior = 0;
-    if (valid && below == 0) prior = atomicAdd(&wcnt[warp][d], __popc(peers));
-    prior = __shfl_sync(kFull, prior, __ffs(peers) - 1);
-    dr[r] = d << 16 | (prior + below);
+    const bool valid = first + r * 32 < n;
+    const uint32_t d = static_cast<uint32_t>(key[r] >> shift) & (kDigits - 1);
+    uint2 *word = &words[warp][d];
+    if (r % kMatchEvery != kMatchEvery - 1) {
+      // every lane sets its bit in its digit's word and reads the word back:
+      // the digit's peers, and its keys before this round.  The lowest peer
+      // moves the count on and clears the bits.
+      if (valid) atomicOr(&word->x, 1u << lane);
+      __syncwarp();
+      const uint2 v = *word;
+      const uint32_t below = __popc(v.x & ((1u << lane) - 1u));
+      dr[r] = valid ? d << 16 | (v.y + below) : kDigits << 16;
+      __syncwarp();
+      if (valid && below == 0) *word = make_uint2(0u, v.y + __popc(v.x));
+      __syncwarp();
+    } else {
+      // the peers by a match; the lowest adds them to the count and hands the
+      // count before them to the others
+      const unsigned peers = __match_any_sync(kFull, valid ? d : static_cast<uint32_t>(kDigits));
+      const uint32_t below = __popc(peers & ((1u << lane) - 1u));
+      uint32_t prior = 0;
+      if (valid && below == 0) {
+        prior = word->y;
+        word->y = prior + __popc(peers);
+      }
+      prior = __shfl_sync(kFull, prior, __ffs(peers) - 1);
+      dr[r] = valid ? d << 16 | (prior + below) : kDigits << 16;
+      __syncwarp();
+    }
   }
   __syncthreads();
   // thread d: digit d's warp prefixes and its count in the tile, then the
@@ -248,9 +277,8 @@ __global__ void __launch_bounds__(kThreads, 4)
   uint32_t cnt = 0;
 #pragma unroll
   for (int w = 0; w < kWarps; w++) {
-    const uint32_t c = wcnt[w][threadIdx.x];
     wcnt[w][threadIdx.x] = cnt;
-    cnt += c;
+    cnt += words[w][threadIdx.x].y;
   }
   uint32_t *mine = nullptr;
   if constexpr (LOOKBACK) {

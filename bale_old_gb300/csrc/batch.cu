@@ -381,7 +381,7 @@ int launch_standalone(const bale_instance_t &x, unsigned long long *bad, void *w
                       cudaStream_t st) {
   if (x.kind == BALE_KIND_IG) {
     if (partition_worthy(x)) return launch_ig_partitioned(x.out, x.in, x.n, x.aux, x.m, x.shift, bad, ws, words, st);
-    return launch_ig(x.out, x.in, x.n, x.aux, x.m, x.shift, bad, st);
+    return launch_ig(x.out, x.in, x.n, x.aux, x.m, x.shift, bad, st, false);
   }
   if (x.kind == BALE_KIND_HISTO) {
     if (bucketed(x)) return launch_histo_bucket(x.out, x.m, x.in, x.n, x.shift, bad, ws, st);

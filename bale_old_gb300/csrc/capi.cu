@@ -150,10 +150,10 @@ void *device_workspace(size_t bytes, cudaStream_t stream) {
   return b.p;
 }
 
-// The bucketed paths' workspaces, most recently used last.  One that a
+// Those workspaces, most recently used last.  One that a
 // captured graph holds is not freed before bale_release_buffers: when it is
-// outgrown or its entry's turn comes it moves to g_bucket_kept.
-struct BucketWs {
+// outgrown or its entry's turn comes it moves to g_call_kept.
+struct CallWs {
   int dev;
   cudaStream_t stream;
   bool captured;
@@ -165,28 +165,28 @@ struct BucketWs {
     captured = false;
   }
 };
-static std::mutex g_bucket_mu;
-static std::vector<BucketWs> g_bucket_ws;
-static std::vector<DevBuf> g_bucket_kept;
+static std::mutex g_call_mu;
+static std::vector<CallWs> g_call_ws;
+static std::vector<DevBuf> g_call_kept;
 
-void *bucket_workspace(size_t bytes, cudaStream_t stream, std::unique_lock<std::mutex> *hold) {
+void *call_workspace(size_t bytes, cudaStream_t stream, std::unique_lock<std::mutex> *hold) {
   const int d = current_device();
   const bool capturing = stream_capturing(stream);
-  *hold = std::unique_lock<std::mutex>(g_bucket_mu);
-  auto it = std::find_if(g_bucket_ws.begin(), g_bucket_ws.end(),
-                         [&](const BucketWs &w) { return w.dev == d && w.stream == stream; });
-  if (it == g_bucket_ws.end()) {
-    if (static_cast<int>(g_bucket_ws.size()) >= kBucketStreams) {
-      g_bucket_ws.front().retire(g_bucket_kept);
-      g_bucket_ws.erase(g_bucket_ws.begin());
+  *hold = std::unique_lock<std::mutex>(g_call_mu);
+  auto it = std::find_if(g_call_ws.begin(), g_call_ws.end(),
+                         [&](const CallWs &w) { return w.dev == d && w.stream == stream; });
+  if (it == g_call_ws.end()) {
+    if (static_cast<int>(g_call_ws.size()) >= kCallStreams) {
+      g_call_ws.front().retire(g_call_kept);
+      g_call_ws.erase(g_call_ws.begin());
     }
-    g_bucket_ws.push_back({d, stream, false, DevBuf()});
+    g_call_ws.push_back({d, stream, false, DevBuf()});
   } else {
-    std::rotate(it, it + 1, g_bucket_ws.end());
+    std::rotate(it, it + 1, g_call_ws.end());
   }
-  BucketWs &w = g_bucket_ws.back();
+  CallWs &w = g_call_ws.back();
   if (bytes > w.buf.cap || !w.buf.p) {
-    w.retire(g_bucket_kept);
+    w.retire(g_call_kept);
     if (cudaMalloc(&w.buf.p, bytes) != cudaSuccess) {
       cudaGetLastError();
       w.buf.p = nullptr;
@@ -699,11 +699,11 @@ void bale_release_buffers(void) {
   std::lock_guard<std::mutex> lk2(g_ws_mu);
   for (auto &kv : g_ws) kv.second.release();
   g_ws.clear();
-  std::lock_guard<std::mutex> lk3(g_bucket_mu);
-  for (auto &w : g_bucket_ws) w.buf.release();
-  g_bucket_ws.clear();
-  for (auto &b : g_bucket_kept) b.release();
-  g_bucket_kept.clear();
+  std::lock_guard<std::mutex> lk3(g_call_mu);
+  for (auto &w : g_call_ws) w.buf.release();
+  g_call_ws.clear();
+  for (auto &b : g_call_kept) b.release();
+  g_call_kept.clear();
 }
 
 int bale_histo_dev(int64_t *d_counts, int64_t ncounts, const int64_t *d_index, int64_t n, int shift,

@@ -26,6 +26,7 @@ int64_t knob_or(const char *name, int64_t dflt);
 // Automatic choice of the region-partitioned kernels (tables beyond L2 with
 // enough elements to amortise the passes); thresholds are tuning knobs.
 bool ig_auto_partition(int64_t n, int64_t table_len);
+bool ig_auto_region(int64_t n, int64_t table_len);
 bool histo_auto_partition(int64_t n, int64_t ncounts);
 // ... and of the histogram by shared-memory buckets.
 bool histo_auto_bucket(int64_t n, int64_t ncounts);
@@ -47,15 +48,16 @@ unsigned long long *next_cursor_words(int k);
 // different streams get their own.  Growing it frees the old buffer, which
 // waits for the device.  Returns nullptr (error set) on allocation failure.
 void *device_workspace(size_t bytes, cudaStream_t stream);
-// The bucketed gather's and histogram's workspaces, apart from the one above:
-// those calls used to need none, so they must not disturb, or be disturbed
-// by, another thread's launches on the same stream.  *hold keeps the pool
+// Workspaces of calls that have a path without one (the bucketed histogram,
+// the region-partitioned gather of middling streams), apart from the one
+// above: such calls must not disturb, or be disturbed by, another thread's
+// launches on the same stream.  *hold keeps the pool
 // locked until the caller has enqueued all of its kernels.  At most
-// kBucketStreams streams keep one; the least recently used one goes first
+// kCallStreams streams keep one; the least recently used one goes first
 // (freeing it waits for the device).  Returns nullptr, with no error set,
 // when there is no memory: the caller then takes a path without one.
-constexpr int kBucketStreams = 8;
-void *bucket_workspace(size_t bytes, cudaStream_t stream, std::unique_lock<std::mutex> *hold);
+constexpr int kCallStreams = 8;
+void *call_workspace(size_t bytes, cudaStream_t stream, std::unique_lock<std::mutex> *hold);
 // Is work on this stream being captured into a graph?
 bool stream_capturing(cudaStream_t stream);
 // The launchers' choices, shared with the batched and serving planners so a
@@ -77,10 +79,10 @@ bool ig_partition_for(int64_t n, int64_t table_len, const int64_t *tgt, const in
   } while (0)
 
 // Launch entry points used by the C ABI (all asynchronous on `stream`).
-// own_ws false: no workspace beyond the plan's own is taken for the bucketed
-// paths (the batch and serving planners account for memory themselves).
+// own_ws false: no call_workspace is taken (the batch and serving planners
+// account for memory themselves).
 int launch_ig(int64_t *tgt, const int64_t *index, int64_t n, const int64_t *table,
-              int64_t table_len, int shift, unsigned long long *bad, cudaStream_t stream);
+              int64_t table_len, int shift, unsigned long long *bad, cudaStream_t stream, bool own_ws = true);
 int launch_histo(int64_t *counts, int64_t ncounts, const int64_t *index, int64_t n, int shift,
                  unsigned long long *bad, cudaStream_t stream, bool own_ws = true);
 int launch_triangle(const int64_t *offset, const int64_t *nonzero, int64_t numrows, int64_t nnz,

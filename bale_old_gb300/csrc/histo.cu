@@ -203,7 +203,7 @@ int launch_histo(int64_t *counts, int64_t ncounts, const int64_t *index, int64_t
   if (mode == 4 && own_ws && stream_capturing(stream)) mode = histo_mode_for(n, ncounts, index, false);
   if (mode == 4) {
     std::unique_lock<std::mutex> hold;
-    void *ws = bucket_workspace(bucket_workspace_bytes(n, ncounts), stream, &hold);
+    void *ws = call_workspace(bucket_workspace_bytes(n, ncounts), stream, &hold);
     if (ws) return launch_histo_bucket(counts, ncounts, index, n, shift, bad, ws, stream);
     mode = histo_auto_partition(n, ncounts) ? 3 : 2;
   }

@@ -13,9 +13,9 @@
 //
 // launch_ig dispatches: this direct gather for tables that fit L2 and for
 // short request streams; for large tables with many requests (the
-// ig.part_min_* knobs) the region-partitioned gather of ig_part.cu, preceded
-// by its device-side skew test, which hands strongly skewed streams back to
-// the direct gather here.
+// ig.part_min_* knobs, and ig_auto_region below them) the region-partitioned
+// gather of ig_part.cu, preceded by its device-side skew test, which hands
+// strongly skewed streams back to the direct gather here.
 #include "common.cuh"
 
 namespace bale {
@@ -168,7 +168,7 @@ namespace {
 
 // The skew test's threshold (knob ig.skew_repeat_pct; 0 turns the test off):
 // the share of sampled requests whose table sector repeats within the sample.
-constexpr int64_t kSkewRepeatPct = 45;
+constexpr int64_t kSkewRepeatPct = 60;
 
 // The direct gather k over n requests, as many blocks as are resident (knob
 // ig.blocks_per_sm overrides) and no more than the work needs.
@@ -193,12 +193,13 @@ int launch_direct(IgKernel k, int threads, int unroll, int64_t *tgt, const int64
 
 bool ig_partition_for(int64_t n, int64_t table_len, const int64_t *tgt, const int64_t *index) {
   const bool aligned = ((reinterpret_cast<uintptr_t>(tgt) | reinterpret_cast<uintptr_t>(index)) & 15) == 0;
+  if (!aligned || !ig_part_supported(n, table_len)) return false;
   const int64_t mode = knob("ig.mode");
-  return aligned && ig_part_supported(n, table_len) && (mode == 1 || (mode < 0 && ig_auto_partition(n, table_len)));
+  return mode == 1 || (mode < 0 && ig_auto_partition(n, table_len));
 }
 
 int launch_ig(int64_t *tgt, const int64_t *index, int64_t n, const int64_t *table,
-              int64_t table_len, int shift, unsigned long long *bad, cudaStream_t stream) {
+              int64_t table_len, int shift, unsigned long long *bad, cudaStream_t stream, bool own_ws) {
   if (n <= 0) return BALE_OK;
   const int sms = num_sms();
   const bool aligned = ((reinterpret_cast<uintptr_t>(tgt) | reinterpret_cast<uintptr_t>(index)) & 15) == 0;
@@ -211,12 +212,10 @@ int launch_ig(int64_t *tgt, const int64_t *index, int64_t n, const int64_t *tabl
       g_l2_fetch_set[dev] = static_cast<int>(fetch + 1);
     }
   }
-  if (ig_partition_for(n, table_len, tgt, index)) {
-    void *ws = device_workspace(ig_part_workspace_bytes(n, table_len), stream);
-    unsigned long long *cursor = next_cursor_word();  // a slot of 4 words: [0] cursor, [1] the skew choice
-    if (!ws || !cursor) return BALE_ENOMEM;
-    // Left to the size rule (ig.mode -1), a skewed stream goes to the direct
-    // gather with L1-allocating table loads instead, chosen on the device.
+  // Through the region partition.  Left to the size rule (ig.mode -1), a
+  // skewed stream goes to the direct gather with L1-allocating table loads
+  // instead, chosen on the device.  cursor: 2 words, [1] for the choice.
+  auto region = [&](void *ws, unsigned long long *cursor) {
     int64_t pct = knob("ig.skew_repeat_pct");
     if (pct < 0) pct = kSkewRepeatPct;
     if (knob("ig.mode") >= 0 || pct == 0 || pct > 100)
@@ -227,6 +226,19 @@ int launch_ig(int64_t *tgt, const int64_t *index, int64_t n, const int64_t *tabl
     if (rc != BALE_OK) return rc;
     return launch_direct(ig_gather_kernel<4, kCached>, 256, 4, tgt, index, n, table, table_len, shift, bad, direct,
                          stream);
+  };
+  if (ig_partition_for(n, table_len, tgt, index)) {
+    void *ws = device_workspace(ig_part_workspace_bytes(n, table_len), stream);
+    unsigned long long *cursor = next_cursor_word();  // a slot of 4 words
+    if (!ws || !cursor) return BALE_ENOMEM;
+    return region(ws, cursor);
+  }
+  if (ig_auto_region(n, table_len) && own_ws && aligned && ig_part_supported(n, table_len) && knob("ig.mode") < 0 &&
+      !stream_capturing(stream)) {
+    std::unique_lock<std::mutex> hold;
+    char *ws = static_cast<char *>(call_workspace(256 + ig_part_workspace_bytes(n, table_len), stream, &hold));
+    if (ws) return region(ws + 256, reinterpret_cast<unsigned long long *>(ws));
+    // no memory for it: the direct gather
   }
   if (!aligned) {
     int64_t want = (n + 255) / 256, full = static_cast<int64_t>(sms) * 8;

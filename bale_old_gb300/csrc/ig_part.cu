@@ -9,8 +9,8 @@
 // exchange happens through HBM in three coalesced passes:
 //
 //  1. partition: each 2048-request chunk is counting-sorted in shared memory
-//     by region (region = 2^21 entries = 16 MiB), whole chunks by a kernel
-//     without per-element bounds checks.  Each request becomes one
+//     by region (region = 2^21 entries = 16 MiB), whole chunks without
+//     per-element bounds checks.  Each request becomes one
 //     u32 (offset in its region << 11 | position in its chunk), written back
 //     grouped by region, plus the chunk's region boundaries (u16);
 //  2. gather: (region, chunk) segments are processed region-major, so at any
@@ -78,16 +78,10 @@ __device__ void block_exclusive_scan(uint32_t *a, int m) {
   __syncthreads();
 }
 
-// Partition of one chunk of any length (the last, partial chunk of a call):
-// chunk c = chunk0 + blockIdx.x.
-__global__ void __launch_bounds__(kThreads)
-    igp_partition_kernel(const int64_t *__restrict__ index, int64_t n, uint64_t tlen, int shift, int nreg,
-                         uint32_t *__restrict__ entries, uint16_t *__restrict__ starts, int64_t chunk0,
-                         const unsigned *__restrict__ direct) {
-  __shared__ uint32_t hist[kMaxRegions + 2];
-  __shared__ __align__(16) uint32_t stage[kChunk];
-  if (direct && *direct) return;
-  const int64_t c = chunk0 + blockIdx.x;
+// Partition of one chunk c of any length (the last, partial chunk of a call).
+__device__ void partition_partial(const int64_t *__restrict__ index, int64_t n, uint64_t tlen, int shift, int nreg,
+                                  uint32_t *__restrict__ entries, uint16_t *__restrict__ starts, int64_t c,
+                                  uint32_t *hist, uint32_t *stage) {
   const int64_t base = c * kChunk;
   const int len = static_cast<int>(n - base < kChunk ? n - base : kChunk);
   for (int i = threadIdx.x; i < nreg + 2; i += kThreads) hist[i] = 0;
@@ -123,14 +117,18 @@ __global__ void __launch_bounds__(kThreads)
 // 62 regions (tables up to 62 * 2^21 entries) one warp scans the counters.
 template <int SHIFT>
 __global__ void __launch_bounds__(kThreads)
-    igp_partition_full_kernel(const int64_t *__restrict__ index, uint64_t tlen, int nreg,
-                              uint32_t *__restrict__ entries, uint16_t *__restrict__ starts,
-                              const unsigned *__restrict__ direct) {
+    igp_partition_kernel(const int64_t *__restrict__ index, int64_t n, uint64_t tlen, int nreg,
+                         uint32_t *__restrict__ entries, uint16_t *__restrict__ starts,
+                         const unsigned *__restrict__ direct) {
   __shared__ uint32_t hist[kMaxRegions + 2];
   __shared__ __align__(16) uint32_t stage[kChunk];  // read back as uint4
   if (direct && *direct) return;
   const int t = threadIdx.x;
   const int64_t c = blockIdx.x;
+  if ((c + 1) * kChunk > n) {
+    partition_partial(index, n, tlen, SHIFT, nreg, entries, starts, c, hist, stage);
+    return;
+  }
   const uint64_t pol = policy_evict_first();
   const longlong2 *src = reinterpret_cast<const longlong2 *>(index + c * kChunk);
   longlong2 v[kPer / 2];
@@ -188,28 +186,55 @@ __global__ void __launch_bounds__(kThreads)
     st_v4_u32_pol(dst + q * kThreads + t, reinterpret_cast<const uint4 *>(stage)[q * kThreads + t], pol);
 }
 
-// Both partition kernels over the n requests: whole chunks, then the partial
-// last one.
 int launch_partition(const int64_t *index, int64_t n, uint64_t tlen, int shift, int nreg, uint32_t *entries,
                      uint16_t *starts, const unsigned *direct, cudaStream_t stream) {
-  const int64_t nfull = n / kChunk;
-  if (nfull > 0) {
-    if (shift == 16)
-      igp_partition_full_kernel<16><<<static_cast<unsigned>(nfull), kThreads, 0, stream>>>(index, tlen, nreg, entries,
-                                                                                        starts, direct);
-    else
-      igp_partition_full_kernel<0><<<static_cast<unsigned>(nfull), kThreads, 0, stream>>>(index, tlen, nreg, entries,
-                                                                                       starts, direct);
-    BALE_CUDA_OK(cudaGetLastError());
-  }
-  if (n % kChunk) {
-    igp_partition_kernel<<<1, kThreads, 0, stream>>>(index, n, tlen, shift, nreg, entries, starts, nfull, direct);
-    BALE_CUDA_OK(cudaGetLastError());
-  }
+  const unsigned blocks = static_cast<unsigned>((n + kChunk - 1) / kChunk);
+  if (shift == 16)
+    igp_partition_kernel<16><<<blocks, kThreads, 0, stream>>>(index, n, tlen, nreg, entries, starts, direct);
+  else
+    igp_partition_kernel<0><<<blocks, kThreads, 0, stream>>>(index, n, tlen, nreg, entries, starts, direct);
+  BALE_CUDA_OK(cudaGetLastError());
   return BALE_OK;
 }
 
-// Segment (region b, chunk c): entries[c*kChunk + s .. c*kChunk + e).
+// The segments (region b, chunk c) in region-major order, entries[c*kChunk + s
+// .. c*kChunk + e).
+__device__ __forceinline__ void gather_segment(const uint32_t *__restrict__ ent, const int64_t *__restrict__ reg,
+                                               int64_t *__restrict__ vo, int s, int e, bool in_table, uint64_t ef,
+                                               unsigned long long &nbad) {
+  const unsigned lane = lane_id();
+  if (in_table) {
+    for (int k = s + static_cast<int>(lane); k < e; k += 128) {
+      uint32_t kk[4];
+      int64_t v[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        kk[u] = (k + 32 * u < e) ? ld_u32_pol(ent + k + 32 * u, ef) : 0u;
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        v[u] = (k + 32 * u < e) ? __ldg(reg + (kk[u] >> kCBits)) : 0;  // may allocate in L1
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (k + 32 * u < e) st_s64_pol(vo + k + 32 * u, v[u], ef);
+    }
+  } else {
+    for (int k = s + static_cast<int>(lane); k < e; k += 32) {
+      st_s64_pol(vo + k, 0, ef);  // out-of-range request: value 0, counted
+      nbad++;
+    }
+  }
+}
+
+// Which segments a warp takes.  Short streams (cursor null): every warps-th
+// segment, so that all warps work on one region, or a few, at a time.  Long
+// ones claim kDescPerClaim segments from a cursor, one claim ahead: a fixed
+// order would let the warps drift over many regions.  A cursor is no use for
+// short streams: claims of 8 segments spread the warps over 8 regions, and
+// claims of one queue on it.  Whole call, 2^26 table entries, us, fixed /
+// claims of 8 / of 1: 20 M requests 253 / 387 / 514, 40 M 458 / 545 / 674,
+// 66 M 783 / 694 / 1392, 2^28 3413 / 2594 / 4923.
+constexpr int64_t kFixedChunks = 20480;  // 42 M requests
+
 __global__ void __launch_bounds__(kThreads)
     igp_gather_kernel(const uint32_t *__restrict__ entries, const uint16_t *__restrict__ starts,
                       int64_t nchunks, int nreg, const int64_t *__restrict__ table,
@@ -218,42 +243,46 @@ __global__ void __launch_bounds__(kThreads)
   if (direct && *direct) return;
   const unsigned lane = lane_id();
   const uint64_t ef = policy_evict_first();
-  const int64_t total = static_cast<int64_t>(nreg + 1) * nchunks;
   unsigned long long nbad = 0;
-  for (;;) {
-    unsigned long long d0 = 0;
-    if (lane == 0) d0 = atomicAdd(cursor, static_cast<unsigned long long>(kDescPerClaim));
-    d0 = __shfl_sync(0xffffffffu, d0, 0);
-    if (static_cast<int64_t>(d0) >= total) break;
-    for (int g = 0; g < kDescPerClaim; g++) {
-      const int64_t d = static_cast<int64_t>(d0) + g;
-      if (d >= total) break;
-      const int b = static_cast<int>(d / nchunks);
-      const int64_t c = d - static_cast<int64_t>(b) * nchunks;
+  if (!cursor) {
+    const int64_t step = static_cast<int64_t>(gridDim.x) * (kThreads / 32);
+    int64_t c = static_cast<int64_t>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5);
+    int b = 0, s = 0, e = 0;
+    // the next segment's bounds load while one is gathered
+    auto settle = [&]() {
+      while (c >= nchunks && b <= nreg) {
+        c -= nchunks;
+        b++;
+      }
+      if (b > nreg) return;
       const uint16_t *st = starts + c * (nreg + 2) + b;
-      const int s = st[0], e = st[1];
-      const uint32_t *ent = entries + c * kChunk;
-      int64_t *vo = val + c * kChunk;
-      if (b < nreg) {
-        const int64_t *reg = table + (static_cast<int64_t>(b) << kRBits);
-        for (int k = s + static_cast<int>(lane); k < e; k += 128) {
-          uint32_t kk[4];
-          int64_t v[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            kk[u] = (k + 32 * u < e) ? ld_u32_pol(ent + k + 32 * u, ef) : 0u;
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            v[u] = (k + 32 * u < e) ? __ldg(reg + (kk[u] >> kCBits)) : 0;  // may allocate in L1
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            if (k + 32 * u < e) st_s64_pol(vo + k + 32 * u, v[u], ef);
-        }
-      } else {
-        for (int k = s + static_cast<int>(lane); k < e; k += 32) {
-          st_s64_pol(vo + k, 0, ef);  // out-of-range request: value 0, counted
-          nbad++;
-        }
+      s = st[0];
+      e = st[1];
+    };
+    settle();
+    while (b <= nreg) {
+      const int b0 = b, s0 = s, e0 = e;
+      const int64_t at = c * kChunk;
+      c += step;
+      settle();
+      gather_segment(entries + at, table + (static_cast<int64_t>(b0) << kRBits), val + at, s0, e0, b0 < nreg, ef, nbad);
+    }
+  } else {
+    const int64_t total = static_cast<int64_t>(nreg + 1) * nchunks;
+    unsigned long long ahead = 0;  // lane 0
+    if (lane == 0) ahead = atomicAdd(cursor, static_cast<unsigned long long>(kDescPerClaim));
+    for (;;) {
+      const int64_t d0 = static_cast<int64_t>(__shfl_sync(0xffffffffu, ahead, 0));
+      if (d0 >= total) break;
+      if (lane == 0) ahead = atomicAdd(cursor, static_cast<unsigned long long>(kDescPerClaim));
+      for (int g = 0; g < kDescPerClaim; g++) {
+        const int64_t d = d0 + g;
+        if (d >= total) break;
+        const int b = static_cast<int>(d / nchunks);
+        const int64_t c = d - static_cast<int64_t>(b) * nchunks, at = c * kChunk;
+        const uint16_t *st = starts + c * (nreg + 2) + b;
+        gather_segment(entries + at, table + (static_cast<int64_t>(b) << kRBits), val + at, st[0], st[1], b < nreg, ef,
+                       nbad);
       }
     }
   }
@@ -335,7 +364,7 @@ __global__ void __launch_bounds__(kThreads)
 // percent of them were: Zipf(s) requests over 2^26 entries repeat 0.04%
 // (uniform), 36% (s = 1.01), 55% (s = 1.1) and 83% (s = 1.3) of an
 // 8192-sample, and the direct gather overtakes the partitioned one between
-// 36% and 55%.
+// 55% and 70%.
 constexpr int kSkewSamples = 8192;
 constexpr int kSkewSlots = 2 * kSkewSamples;  // the set is never more than half full
 constexpr int kSkewThreads = 1024;
@@ -457,18 +486,18 @@ int launch_ig_partitioned(int64_t *tgt, const int64_t *index, int64_t n, const i
   p += static_cast<size_t>(nchunks) * kChunk * sizeof(int64_t);
   uint16_t *starts = reinterpret_cast<uint16_t *>(p);
 
-  BALE_CUDA_OK(cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), stream));
+  if (nchunks > kFixedChunks) BALE_CUDA_OK(cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), stream));
   int rc = launch_partition(index, n, static_cast<uint64_t>(table_len), shift, nreg, entries, starts, direct, stream);
   if (rc != BALE_OK) return rc;
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, igp_gather_kernel, kThreads, 0) != cudaSuccess || occ < 1)
     occ = 1;
   int64_t blocks = static_cast<int64_t>(num_sms()) * occ;
-  const int64_t warps_needed = ((nreg + 1) * nchunks + kDescPerClaim - 1) / kDescPerClaim;
+  const int64_t warps_needed = (nreg + 1) * nchunks;
   if (blocks * (kThreads / 32) > warps_needed) blocks = (warps_needed + (kThreads / 32) - 1) / (kThreads / 32);
   if (blocks < 1) blocks = 1;
-  igp_gather_kernel<<<static_cast<unsigned>(blocks), kThreads, 0, stream>>>(entries, starts, nchunks, nreg,
-                                                                          table, val, cursor, bad, direct);
+  igp_gather_kernel<<<static_cast<unsigned>(blocks), kThreads, 0, stream>>>(
+      entries, starts, nchunks, nreg, table, val, nchunks <= kFixedChunks ? nullptr : cursor, bad, direct);
   BALE_CUDA_OK(cudaGetLastError());
   igp_unpermute_kernel<<<static_cast<unsigned>(nchunks), kThreads, 0, stream>>>(entries, val, tgt, n, direct);
   BALE_CUDA_OK(cudaGetLastError());

@@ -96,6 +96,15 @@ bool ig_auto_partition(int64_t n, int64_t table_len) {
          n >= knob_or("ig.part_min_requests", int64_t(1) << 20);
 }
 
+// Streams that the knobs leave to the direct gather, over a table well beyond
+// L2: the region partition pays from 8 M requests (uniform, us, direct /
+// partitioned: 2^26 entries 4 M 95 / 105, 8 M 187 / 160, 20 M 460 / 253; 2^25
+// entries 4 M 75 / 93, 8 M 146 / 134, 20 M 357 / 262; 2^24 entries 20 M 226 /
+// 234, 66 M 728 / 704).
+bool ig_auto_region(int64_t n, int64_t table_len) {
+  return n >= int64_t(8) << 20 && table_len >= int64_t(1) << 25;
+}
+
 bool histo_auto_partition(int64_t n, int64_t ncounts) {
   return ncounts * 8 > knob_or("histo.part_min_table_bytes", int64_t(96) << 20) &&
          n >= knob_or("histo.part_min_updates", int64_t(1) << 20);

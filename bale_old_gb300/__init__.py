@@ -246,7 +246,9 @@ def _stream(stream) -> int:
     if stream is None:
         import torch
 
-        return torch.cuda.current_stream().cuda_stream
+        # the current stream's handle without a Stream object around it, which
+        # costs 3 us, a third of a small call
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
     return int(getattr(stream, "cuda_stream", stream))
 
 

@@ -116,6 +116,11 @@ bool bucket_supported(int64_t n, int64_t ncounts);
 size_t bucket_workspace_bytes(int64_t n, int64_t ncounts);
 int launch_histo_bucket(int64_t *counts, int64_t ncounts, const int64_t *index, int64_t n, int shift,
                         unsigned long long *bad, void *ws, cudaStream_t stream);
+// The same for the degrees of *nkeys (at most `most`) edge keys a << S | b:
+// deg[a]++, deg[b]++, with a workspace of 8 * most bytes (256-byte aligned).
+bool degrees_bucket_supported(int64_t most, int64_t n);
+int launch_degrees_bucket(uint32_t *deg, int64_t n, const uint64_t *keys, const unsigned *nkeys, int64_t most, int S,
+                          void *ws, cudaStream_t stream);
 // Bitmap/search hybrid triangle counting (tri_hybrid.cu); needs numrows < 2^32.
 size_t tri_hybrid_workspace_bytes(int64_t numrows, int64_t nnz);
 // run_if (optional, here and in the wedge functions below): a device word;

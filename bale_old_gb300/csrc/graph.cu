@@ -5,10 +5,11 @@
 // bale_gen_rmat in host/inputs.c):
 //   1. keys: each edge {u,v}, u != v, becomes min << S | max (S = label
 //      bits); self loops become an all-ones key that sorts last;
-//   2. sort the keys (LSD radix sort), drop the duplicates and the
-//      self loops;
-//   3. degrees; labels by descending degree, ties by ascending original
-//      label: a second sort of (maxdeg - deg) << S | v;
+//   2. the distinct keys and the degrees: for 2^20 to 2^26 edges by hashing
+//      (graph_unique.cu), else by sorting the keys (LSD radix sort) and
+//      dropping the duplicates and the self loops;
+//   3. labels by descending degree, ties by ascending original label: a stable
+//      sort of (maxdeg - deg) << S | v on the degree's bits;
 //   4. each edge relabelled to row = max, col = min of the new labels, a
 //      third sort, and the CSR read off the sorted keys: rows in order,
 //      columns ascending within each row -- the reference's tidy lower
@@ -169,38 +170,66 @@ uint32_t prob_threshold(double p) {
 }
 
 
-// Steps 2-4 from the edge keys in w.ka (m of them).
-int build_from_keys(Ws &w, int64_t m, int64_t n, int S, int64_t *d_offset, int64_t *d_nonzero, int64_t *nnz,
-                    cudaStream_t st) {
+// The distinct edge keys of the m in w.ka by sorting, into *unique (one of w.ka
+// and w.kb, *other the other), their number into w.words[0], and the degrees.
+int unique_by_sort(Ws &w, int64_t m, int64_t n, int S, uint64_t **unique, uint64_t **other, cudaStream_t st) {
   int rc = BALE_OK;
   const int kbits = std::min(64, 2 * S + 1);
   uint64_t *sorted = radix_sort(w.ka, w.kb, m, kbits, w, st, &rc);
   if (rc != BALE_OK) return rc;
-  uint64_t *other = sorted == w.ka ? w.kb : w.ka;
+  *unique = sorted == w.ka ? w.kb : w.ka;
+  *other = sorted;
   unique_flag_kernel<<<grid_for(m), 256, 0, st>>>(sorted, m, S, w.flag);
   rc = excl_scan(w.flag, w.pos, m, w.bsum, w.words, st);
   if (rc != BALE_OK) return rc;
   BALE_CUDA_OK(cudaMemsetAsync(w.deg, 0, static_cast<size_t>(n) * 4, st));
   // few blocks: each flushes its kHubIds shared counters at the end
   compact_degree_kernel<<<std::min<unsigned>(grid_for(m), num_sms() * 4), 256, 0, st>>>(sorted, m, S, n, w.flag,
-                                                                                    w.pos, other, w.deg);
-  unsigned int nu32 = 0;
-  BALE_CUDA_OK(cudaMemcpyAsync(&nu32, w.words, 4, cudaMemcpyDeviceToHost, st));
-  BALE_CUDA_OK(cudaMemsetAsync(w.words + 1, 0, 4, st));
+                                                                                    w.pos, *unique, w.deg);
+  BALE_CUDA_OK(cudaGetLastError());
+  return BALE_OK;
+}
+
+// The largest degree into w.words[1]; both it and the number of distinct
+// edges (w.words[0]) on the host.
+int read_sizes(Ws &w, int64_t n, unsigned int size[4], cudaStream_t st) {
   max_kernel<<<grid_for(n), 256, 0, st>>>(w.deg, n, w.words + 1);
-  unsigned int maxdeg = 0;
-  BALE_CUDA_OK(cudaMemcpyAsync(&maxdeg, w.words + 1, 4, cudaMemcpyDeviceToHost, st));
+  BALE_CUDA_OK(cudaMemcpyAsync(size, w.words, 4 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
   BALE_CUDA_OK(cudaStreamSynchronize(st));
-  const int64_t nu = nu32;
+  return BALE_OK;
+}
+
+// Steps 2-4 from the edge keys in w.ka (m of them; w.words zero before).
+int build_from_keys(Ws &w, int64_t m, int64_t n, int S, int64_t *d_offset, int64_t *d_nonzero, int64_t *nnz,
+                    cudaStream_t st) {
+  int rc = BALE_OK;
+  unsigned int size[4] = {0, 0, 0, 0};
+  uint64_t *other = w.ka, *sorted = w.kb;  // the unique keys, and a buffer for the lower keys
+  const bool hashed = unique_edges_supported(m, n);
+  if (hashed) {
+    if ((rc = unique_edges(w, m, n, S, w.words, st)) != BALE_OK) return rc;
+    if ((rc = read_sizes(w, n, size, st)) != BALE_OK) return rc;
+  }
+  if (!hashed || size[2]) {
+    if (hashed) {
+      std::swap(w.ka, w.kb);
+      m = size[3];
+    }
+    BALE_CUDA_OK(cudaMemsetAsync(w.words, 0, 4 * sizeof(unsigned int), st));
+    if ((rc = unique_by_sort(w, m, n, S, &other, &sorted, st)) != BALE_OK) return rc;
+    if ((rc = read_sizes(w, n, size, st)) != BALE_OK) return rc;
+  }
+  const int64_t nu = size[0];
+  const unsigned int maxdeg = size[1];
   vertex_keys_kernel<<<grid_for(n), 256, 0, st>>>(w.deg, n, S, w.words + 1, w.va);
   int dbits = 1;
   while ((uint64_t(1) << dbits) <= maxdeg) dbits++;
-  uint64_t *vs = radix_sort(w.va, w.vb, n, std::min(64, S + dbits), w, st, &rc);
+  // by degree alone: the vertices start in label order and the sort is stable
+  uint64_t *vs = radix_sort(w.va, w.vb, n, std::min(64, S + dbits), w, st, &rc, S);
   if (rc != BALE_OK) return rc;
   new_label_kernel<<<grid_for(n), 256, 0, st>>>(vs, n, S, w.newid);
-  uint64_t *lk = sorted;  // the unique keys are in `other`; reuse `sorted` for the lower keys
-  lower_keys_kernel<<<grid_for(nu), 256, 0, st>>>(other, nu, S, w.newid, lk);
-  uint64_t *ls = radix_sort(lk, other, nu, 2 * S, w, st, &rc);
+  lower_keys_kernel<<<grid_for(nu), 256, 0, st>>>(other, nu, S, w.newid, sorted);
+  uint64_t *ls = radix_sort(sorted, other, nu, 2 * S, w, st, &rc);
   if (rc != BALE_OK) return rc;
   rc = csr_from_keys(ls, nu, n, S, d_offset, d_nonzero, st);
   if (rc != BALE_OK) return rc;

@@ -1,0 +1,266 @@
+// graph_unique.cu -- the distinct edges of a large edge list, and the degrees,
+// without sorting it.
+//
+// The graph build needs each undirected edge once, in any order: the labels
+// come from the degrees, and the matrix is ordered afterwards.  Sorting the
+// keys to find the repeats takes a pass over them per 8 bits.  Here a hash of
+// the key picks one of up to 16384 buckets of about 4096 keys:
+//
+//  1. count the keys of every bucket (self loops are dropped here);
+//  2. partition: each chunk of 8192 keys is counting-sorted by bucket in shared
+//     memory and its runs appended to the buckets (one atomic per bucket and
+//     chunk reserves the place);
+//  3. unique: a CTA per bucket puts the keys into a hash set in shared memory;
+//     each key that was not there yet is kept.
+//
+// The degrees are a histogram of the endpoints, taken by shared-memory buckets
+// (histo_bucket.cu); reductions at L2 from step 3 made it 340 us slower for
+// 2^24 edges, queueing on the hubs.
+//
+// 2^24 R-MAT edges, 2^20 vertices, us: count 27, partition 139 (bound by its
+// shared-memory accesses and the stores of runs of two keys), unique 101,
+// degrees 105; sorting the keys, flagging, scanning and compacting with degrees
+// took 1000.  Below 2^20 edges the sort stays (its passes are launches there),
+// and above 2^26, where a bucket would outgrow its set.
+//
+// Equal keys meet in one bucket, so a bucket's set holds its distinct keys
+// only.  A bucket with more distinct keys than its set takes (the hash spreads
+// them evenly, so only keys made for it have one) raises a flag, and the caller
+// sorts the keys after all.
+#include <algorithm>
+
+#include "sort.cuh"
+
+namespace bale {
+namespace {
+
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kThreads = 512;
+constexpr int kPer = 16;
+constexpr int kChunk = kThreads * kPer;  // keys per partition chunk and per round of a bucket: 8192
+constexpr int kMaxBits = 14;             // log2 of the buckets
+constexpr int kSetBits = 13;
+constexpr int kSet = 1 << kSetBits;      // places of a bucket's hash set: 64 KiB
+constexpr int kProbes = 256;             // places tried before a key does not fit
+constexpr int kSetThreads = 512;
+constexpr int kSetPer = 8;
+constexpr uint64_t kNone = ~uint64_t(0);  // no key: an empty place, or a self loop in the key array
+
+// All bits of the key in the top ones (the bucket) and in the middle (the
+// place): two rounds of multiply and fold.
+__device__ __forceinline__ uint64_t mix(uint64_t k) {
+  k *= 0x9E3779B97F4A7C15ull;
+  k ^= k >> 32;
+  return k * 0xD6E8FEB86659FD93ull;
+}
+
+__device__ __forceinline__ uint32_t bucket_of(uint64_t k, int bits) {
+  return bits ? static_cast<uint32_t>(mix(k) >> (64 - bits)) : 0u;
+}
+
+__device__ __forceinline__ uint32_t incl_scan_u32(uint32_t v) {
+  const unsigned lane = lane_id();
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, v, o);
+    if (static_cast<int>(lane) >= o) v += y;
+  }
+  return v;
+}
+
+// Exclusive scan of a[0,m) in shared memory, in place, by a block of THREADS.
+template <int THREADS>
+__device__ __forceinline__ void block_scan(uint32_t *a, int m, uint32_t *warp_tot) {
+  const int per = (m + THREADS - 1) / THREADS, lo = min(static_cast<int>(threadIdx.x) * per, m), hi = min(lo + per, m);
+  uint32_t sum = 0;
+  for (int i = lo; i < hi; i++) sum += a[i];
+  const uint32_t inc = incl_scan_u32(sum);
+  if (lane_id() == 31) warp_tot[threadIdx.x >> 5] = inc;
+  __syncthreads();
+  uint32_t run = inc - sum;
+  for (unsigned w = 0; w < (threadIdx.x >> 5); w++) run += warp_tot[w];
+  for (int i = lo; i < hi; i++) {
+    const uint32_t v = a[i];
+    a[i] = run;
+    run += v;
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(kThreads)
+    unique_count_kernel(const uint64_t *__restrict__ keys, int64_t m, int bits, uint32_t *__restrict__ count) {
+  extern __shared__ uint32_t hist[];
+  const int nb = 1 << bits;
+  for (int i = threadIdx.x; i < nb; i += kThreads) hist[i] = 0;
+  __syncthreads();
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * kThreads;
+  int64_t e = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
+  for (; e + 3 * stride < m; e += 4 * stride) {
+    uint64_t k[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) k[u] = keys[e + u * stride];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (k[u] != kNone) atomicAdd(&hist[bucket_of(k[u], bits)], 1u);
+  }
+  for (; e < m; e += stride) {
+    const uint64_t k = keys[e];
+    if (k != kNone) atomicAdd(&hist[bucket_of(k, bits)], 1u);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nb; i += kThreads)
+    if (hist[i]) atomicAdd(count + i, hist[i]);
+}
+
+// count[0, nb) becomes the buckets' starts, count[nb] and *total the number of
+// keys, and next a copy of the starts.
+__global__ void __launch_bounds__(1024)
+    unique_starts_kernel(uint32_t *__restrict__ count, uint32_t *__restrict__ next, int nb,
+                         unsigned int *__restrict__ total) {
+  extern __shared__ uint32_t a[];
+  __shared__ uint32_t warp_tot[32];
+  for (int i = threadIdx.x; i <= nb; i += 1024) a[i] = i < nb ? count[i] : 0u;
+  __syncthreads();
+  block_scan<1024>(a, nb + 1, warp_tot);
+  for (int i = threadIdx.x; i <= nb; i += 1024) {
+    count[i] = a[i];
+    if (i < nb) next[i] = a[i];
+    else *total = a[i];
+  }
+}
+
+__global__ void __launch_bounds__(kThreads)
+    unique_partition_kernel(const uint64_t *__restrict__ keys, int64_t m, int bits, uint32_t *__restrict__ next,
+                            uint64_t *__restrict__ out) {
+  extern __shared__ __align__(16) uint64_t stage[];  // kChunk keys, then the buckets' places and shifts
+  __shared__ uint32_t warp_tot[kThreads / 32], total;
+  const int nb = 1 << bits, t = threadIdx.x;
+  uint32_t *hist = reinterpret_cast<uint32_t *>(stage + kChunk), *shift = hist + nb;
+  for (int i = t; i < nb; i += kThreads) hist[i] = 0;
+  __syncthreads();
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * kChunk;
+  uint64_t key[kPer];
+  uint32_t rank[kPer / 2];  // two 16-bit ranks each
+#pragma unroll
+  for (int r = 0; r < kPer; r++) key[r] = base + r * kThreads + t < m ? keys[base + r * kThreads + t] : kNone;
+#pragma unroll
+  for (int r = 0; r < kPer; r++) {
+    uint32_t x = 0;
+    if (key[r] != kNone) x = atomicAdd(&hist[bucket_of(key[r], bits)], 1u);
+    rank[r / 2] = r % 2 ? rank[r / 2] | x << 16 : x;
+  }
+  __syncthreads();
+  // each bucket's run: its place in the output, less its place in the chunk
+  for (int i = t; i < nb; i += kThreads) shift[i] = hist[i] ? atomicAdd(next + i, hist[i]) : 0u;
+  if (t == 0) total = 0;
+  __syncthreads();
+  uint32_t mine = 0;
+#pragma unroll
+  for (int r = 0; r < kPer; r++) mine += key[r] != kNone;
+  block_scan<kThreads>(hist, nb, warp_tot);
+  for (int i = t; i < nb; i += kThreads) shift[i] -= hist[i];
+  mine = __reduce_add_sync(kFull, mine);
+  if (lane_id() == 0) atomicAdd(&total, mine);
+#pragma unroll
+  for (int r = 0; r < kPer; r++)
+    if (key[r] != kNone)
+      stage[hist[bucket_of(key[r], bits)] + (r % 2 ? rank[r / 2] >> 16 : rank[r / 2] & 0xffffu)] = key[r];
+  __syncthreads();
+  for (uint32_t i = t; i < total; i += kThreads) {
+    const uint64_t k = stage[i];
+    out[shift[bucket_of(k, bits)] + i] = k;
+  }
+}
+
+__global__ void __launch_bounds__(kSetThreads)
+    unique_set_kernel(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ starts,
+                      uint64_t *__restrict__ out, unsigned int *__restrict__ nout,
+                      unsigned int *__restrict__ overflow) {
+  extern __shared__ __align__(16) unsigned long long set[];
+  __shared__ uint32_t warp_new[kSetThreads / 32], first;
+  const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+  const uint32_t lo = starts[blockIdx.x], hi = starts[blockIdx.x + 1];
+  if (lo == hi) return;
+  for (int i = threadIdx.x; i < kSet / 2; i += kSetThreads)
+    reinterpret_cast<ulonglong2 *>(set)[i] = make_ulonglong2(kNone, kNone);
+  __syncthreads();
+  for (uint32_t r0 = lo; r0 < hi; r0 += kSetThreads * kSetPer) {
+    uint64_t key[kSetPer];
+    uint32_t fresh = 0;
+#pragma unroll
+    for (int r = 0; r < kSetPer; r++) {
+      const uint32_t i = r0 + r * kSetThreads + threadIdx.x;
+      key[r] = i < hi ? keys[i] : kNone;
+    }
+#pragma unroll
+    for (int r = 0; r < kSetPer; r++) {
+      if (key[r] == kNone) continue;
+      uint32_t h = static_cast<uint32_t>(mix(key[r]) >> 24) & (kSet - 1);
+      int probe = 0;
+      for (; probe < kProbes; probe++) {
+        const unsigned long long old = atomicCAS(set + h, kNone, static_cast<unsigned long long>(key[r]));
+        if (old == kNone) fresh |= 1u << r;
+        if (old == kNone || old == key[r]) break;
+        h = (h + 1) & (kSet - 1);
+      }
+      if (probe == kProbes) *overflow = 1;
+    }
+    // the new keys, side by side
+    uint32_t n = 0;
+#pragma unroll
+    for (int r = 0; r < kSetPer; r++) n += __popc(__ballot_sync(kFull, fresh >> r & 1u));
+    if (lane == 0) warp_new[warp] = n;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t sum = 0;
+      for (int w = 0; w < kSetThreads / 32; w++) {
+        const uint32_t x = warp_new[w];
+        warp_new[w] = sum;
+        sum += x;
+      }
+      first = atomicAdd(nout, sum);
+    }
+    __syncthreads();
+    uint32_t at = first + warp_new[warp];
+#pragma unroll
+    for (int r = 0; r < kSetPer; r++) {
+      const bool f = fresh >> r & 1u;
+      const unsigned b = __ballot_sync(kFull, f);
+      if (f) out[at + __popc(b & ((1u << lane) - 1u))] = key[r];
+      at += __popc(b);
+    }
+    __syncthreads();
+  }
+}
+
+}  // namespace
+
+bool unique_edges_supported(int64_t m, int64_t n) {
+  return m >= (int64_t(1) << 20) && m <= (int64_t(1) << 26) && degrees_bucket_supported(m, n);
+}
+
+int unique_edges(Ws &w, int64_t m, int64_t n, int S, unsigned int *words, cudaStream_t st) {
+  int bits = 0;
+  while (bits < kMaxBits && (m >> bits) > (bits < 10 ? 512 : 4096)) bits++;
+  const int nb = 1 << bits;
+  uint32_t *count = w.hist, *next = w.hoff;
+  BALE_CUDA_OK(cudaMemsetAsync(count, 0, static_cast<size_t>(nb + 1) * 4, st));
+  BALE_CUDA_OK(cudaMemsetAsync(w.deg, 0, static_cast<size_t>(n) * 4, st));
+  const int csmem = nb * 4, ssmem = (nb + 1) * 4, psmem = kChunk * 8 + nb * 8, usmem = kSet * 8;
+  BALE_CUDA_OK(cudaFuncSetAttribute(unique_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, csmem));
+  BALE_CUDA_OK(cudaFuncSetAttribute(unique_starts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ssmem));
+  BALE_CUDA_OK(cudaFuncSetAttribute(unique_partition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem));
+  BALE_CUDA_OK(cudaFuncSetAttribute(unique_set_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, usmem));
+  const int64_t per_sm = bits > 12 ? 3 : 4;
+  const unsigned cblocks = static_cast<unsigned>(
+      std::min<int64_t>((m + kThreads - 1) / kThreads, static_cast<int64_t>(num_sms()) * per_sm));
+  unique_count_kernel<<<cblocks, kThreads, csmem, st>>>(w.ka, m, bits, count);
+  unique_starts_kernel<<<1, 1024, ssmem, st>>>(count, next, nb, words + 3);
+  unique_partition_kernel<<<static_cast<unsigned>((m + kChunk - 1) / kChunk), kThreads, psmem, st>>>(w.ka, m, bits,
+                                                                                                  next, w.kb);
+  unique_set_kernel<<<nb, kSetThreads, usmem, st>>>(w.kb, count, w.ka, words, words + 2);
+  BALE_CUDA_OK(cudaGetLastError());
+  return launch_degrees_bucket(w.deg, n, w.ka, words, m, S, w.flag, st);  // flag and pos lie together
+}
+
+}  // namespace bale

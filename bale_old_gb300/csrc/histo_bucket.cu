@@ -105,8 +105,13 @@ __device__ __forceinline__ void block_scan(uint32_t *a, int m, uint32_t *warp_to
   __syncthreads();
 }
 
-template <int SHIFT, bool WHOLE>
-__device__ __forceinline__ void partition_chunk(const int64_t *__restrict__ index, int64_t n, uint64_t ncounts,
+// What an update stream is made of: 64-bit indices to be shifted right by SRC
+// (0 or 16), or, for the degrees of a graph, edge keys a << S | b with two
+// updates each.
+constexpr int kEdges = -1;
+
+template <int SRC, bool WHOLE>
+__device__ __forceinline__ void partition_chunk(const int64_t *__restrict__ index, int64_t n, uint64_t ncounts, int S,
                                                 Buckets bk, uint16_t *__restrict__ off16,
                                                 uint16_t *__restrict__ starts, uint32_t *__restrict__ words,
                                                 unsigned long long *__restrict__ bad, uint32_t *hist, uint16_t *stage,
@@ -118,24 +123,32 @@ __device__ __forceinline__ void partition_chunk(const int64_t *__restrict__ inde
   for (int i = t; i < nb + 2; i += kPartThreads) hist[i] = 0;
   __syncthreads();
   uint32_t key[kPer];  // bucket << 16 | offset in the bucket; bucket nb for an out-of-range update
-  const longlong2 *src = reinterpret_cast<const longlong2 *>(index + base);
+  constexpr int kEach = SRC == kEdges ? 4 : 2;  // updates of a 16-byte vector
+  const longlong2 *src = reinterpret_cast<const longlong2 *>(SRC == kEdges ? index + base / 2 : index + base);
+  const int64_t *src1 = reinterpret_cast<const int64_t *>(src);
 #pragma unroll
-  for (int h = 0; h < kPer / 2; h++) {
+  for (int h = 0; h < kPer / kEach; h++) {
     longlong2 v;
-    const int e0 = 2 * (h * kPartThreads + t);  // position in the chunk of v.x
+    const int at = h * kPartThreads + t;  // the vector's place in the chunk
     if (WHOLE) {
-      v = ld_v2_s64_pol(src + h * kPartThreads + t, pol);
+      v = ld_v2_s64_pol(src + at, pol);
     } else {
-      v.x = e0 < len ? index[base + e0] : 0;
-      v.y = e0 + 1 < len ? index[base + e0 + 1] : 0;
+      v.x = at * kEach < len ? src1[2 * at] : 0;
+      v.y = at * kEach + kEach / 2 < len ? src1[2 * at + 1] : 0;
     }
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-      const uint64_t k = static_cast<uint64_t>((j ? v.y : v.x) >> SHIFT);
+    for (int j = 0; j < kEach; j++) {
+      uint64_t k;
+      if constexpr (SRC == kEdges) {
+        const uint64_t e = static_cast<uint64_t>(j < 2 ? v.x : v.y);
+        k = j % 2 ? e & ((uint64_t(1) << S) - 1) : e >> S;
+      } else {
+        k = static_cast<uint64_t>((j ? v.y : v.x) >> SRC);
+      }
       const uint32_t k32 = static_cast<uint32_t>(k), b = bucket_of(k32, bk);
       const uint32_t kk = k < ncounts ? (b << 16 | (k32 - b * bk.size)) : static_cast<uint32_t>(nb) << 16;
-      key[2 * h + j] = kk;
-      if (WHOLE || e0 + j < len) atomicAdd(&hist[kk >> 16], 1u);
+      key[kEach * h + j] = kk;
+      if (WHOLE || at * kEach + j < len) atomicAdd(&hist[kk >> 16], 1u);
     }
   }
   __syncthreads();
@@ -146,11 +159,11 @@ __device__ __forceinline__ void partition_chunk(const int64_t *__restrict__ inde
     starts[start_at(c, i, nb + 2)] = static_cast<uint16_t>(at);
     if (counted && i < nb) atomicAdd(words + kWordTotals + i, hist[i + 1] - at);
   }
-  if (t == 0 && hist[nb + 1] != hist[nb]) atomicAdd(bad, static_cast<unsigned long long>(hist[nb + 1] - hist[nb]));
+  if (t == 0 && bad && hist[nb + 1] != hist[nb]) atomicAdd(bad, static_cast<unsigned long long>(hist[nb + 1] - hist[nb]));
   __syncthreads();
 #pragma unroll
   for (int s = 0; s < kPer; s++)
-    if (WHOLE || 2 * ((s >> 1) * kPartThreads + t) + (s & 1) < len)
+    if (WHOLE || kEach * ((s / kEach) * kPartThreads + t) + s % kEach < len)
       stage[atomicAdd(&hist[key[s] >> 16], 1u)] = static_cast<uint16_t>(key[s]);
   __syncthreads();
   // a partial chunk's last vector carries unused entries (off16 holds whole chunks)
@@ -158,18 +171,23 @@ __device__ __forceinline__ void partition_chunk(const int64_t *__restrict__ inde
   for (int i = t; i < (len + 7) / 8; i += kPartThreads) o[i] = reinterpret_cast<const uint4 *>(stage)[i];
 }
 
-template <int SHIFT>
+// n_dev (edges): the number of keys, known to the device only; n is then the
+// most it can be.
+template <int SRC>
 __global__ void __launch_bounds__(kPartThreads, kPartBlocks)
-    bucket_partition_kernel(const int64_t *__restrict__ index, int64_t n, uint64_t ncounts, Buckets bk,
-                            uint16_t *__restrict__ off16, uint16_t *__restrict__ starts, uint32_t *__restrict__ words,
+    bucket_partition_kernel(const int64_t *__restrict__ index, int64_t n, const unsigned *__restrict__ n_dev,
+                            uint64_t ncounts, int S, Buckets bk, uint16_t *__restrict__ off16,
+                            uint16_t *__restrict__ starts, uint32_t *__restrict__ words,
                             unsigned long long *__restrict__ bad) {
   extern __shared__ __align__(16) uint16_t stage[];  // kChunk entries, then nb + 2 counts
   __shared__ uint32_t warp_tot[kPartThreads / 32];
   uint32_t *hist = reinterpret_cast<uint32_t *>(stage + kChunk);
+  if constexpr (SRC == kEdges) n = 2 * static_cast<int64_t>(*n_dev);
+  if (static_cast<int64_t>(blockIdx.x) * kChunk >= n) return;
   if ((static_cast<int64_t>(blockIdx.x) + 1) * kChunk <= n)
-    partition_chunk<SHIFT, true>(index, n, ncounts, bk, off16, starts, words, bad, hist, stage, warp_tot);
+    partition_chunk<SRC, true>(index, n, ncounts, S, bk, off16, starts, words, bad, hist, stage, warp_tot);
   else
-    partition_chunk<SHIFT, false>(index, n, ncounts, bk, off16, starts, words, bad, hist, stage, warp_tot);
+    partition_chunk<SRC, false>(index, n, ncounts, S, bk, off16, starts, words, bad, hist, stage, warp_tot);
 }
 
 // The items: bucket b is cut into parts(b) = its sampled requests * scale,
@@ -305,13 +323,20 @@ __device__ __forceinline__ void count_group(const uint4 *__restrict__ ent, uint3
   }
 }
 
+__device__ __forceinline__ void add_count(int64_t *p, uint32_t v) { red_add_u64(p, v); }
+__device__ __forceinline__ void add_count(uint32_t *p, uint32_t v) { atomicAdd(p, v); }
+
+// Counter: the table's type.  n_dev as in the partition.
+template <class Counter>
 __global__ void __launch_bounds__(kCountThreads, kCountBlocks)
     bucket_count_kernel(const uint16_t *__restrict__ off16, const uint16_t *__restrict__ starts, int64_t nchunks,
-                        Buckets bk, float scale, int64_t *__restrict__ counts, uint64_t ncounts,
-                        uint32_t *__restrict__ words) {
+                        const unsigned *__restrict__ n_dev, Buckets bk, float scale, Counter *__restrict__ counts,
+                        uint64_t ncounts, uint32_t *__restrict__ words) {
   extern __shared__ __align__(16) uint32_t cnts[];  // bk.size counters rounded up to 4, then the item plan
   __shared__ uint32_t warp_tot[kCountThreads / 32], post[2];
   const uint32_t cnts_at = static_cast<uint32_t>(__cvta_generic_to_shared(cnts));
+  if (n_dev) nchunks = (2 * static_cast<int64_t>(*n_dev) + kChunk - 1) / kChunk;
+  if (nchunks == 0) return;
   const uint32_t nch = static_cast<uint32_t>(nchunks), quads = (bk.size + 3u) / 4u;
   uint16_t *ends = reinterpret_cast<uint16_t *>(cnts + quads * 4u);
   const uint32_t items = plan_items<kCountThreads>(words, bk.n, scale, nch, ends, warp_tot);
@@ -344,7 +369,7 @@ __global__ void __launch_bounds__(kCountThreads, kCountBlocks)
 #pragma unroll 4
     for (uint32_t i = threadIdx.x; i < have; i += kCountThreads) {
       const uint32_t v = cnts[i];
-      if (v) red_add_u64(counts + t0 + i, v);
+      if (v) add_count(counts + t0 + i, v);
     }
     __syncthreads();
   }
@@ -402,26 +427,54 @@ bool bucket_supported(int64_t n, int64_t ncounts) {
 
 size_t bucket_workspace_bytes(int64_t n, int64_t ncounts) { return layout(n, ncounts).total; }
 
+namespace {
+
+// Both kernels.
+template <int SRC, class Counter>
+int launch(Counter *counts, int64_t ncounts, const int64_t *index, int64_t n, const unsigned *n_dev, int S,
+           unsigned long long *bad, const Layout &l, uint32_t *words, uint16_t *starts, uint16_t *off16,
+           cudaStream_t stream) {
+  BALE_CUDA_OK(cudaMemsetAsync(words, 0, l.words_bytes, stream));
+  auto part = bucket_partition_kernel<SRC>;
+  const int psmem = kChunk * 2 + (l.bk.n + 2) * 4;
+  BALE_CUDA_OK(cudaFuncSetAttribute(part, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem));
+  part<<<static_cast<unsigned>(l.nchunks), kPartThreads, psmem, stream>>>(
+      index, n, n_dev, static_cast<uint64_t>(ncounts), S, l.bk, off16, starts, words, bad);
+  BALE_CUDA_OK(cudaGetLastError());
+  auto count = bucket_count_kernel<Counter>;
+  const int csmem = static_cast<int>((l.bk.size + 3) / 4 * 16 + l.bk.n * 2);
+  BALE_CUDA_OK(cudaFuncSetAttribute(count, cudaFuncAttributeMaxDynamicSharedMemorySize, csmem));
+  const int64_t slots = walk_slots();
+  count<<<static_cast<unsigned>(slots), kCountThreads, csmem, stream>>>(
+      off16, starts, l.nchunks, n_dev, l.bk, part_scale(n, l.bk, slots), counts, static_cast<uint64_t>(ncounts), words);
+  BALE_CUDA_OK(cudaGetLastError());
+  return BALE_OK;
+}
+
+}  // namespace
+
 int launch_histo_bucket(int64_t *counts, int64_t ncounts, const int64_t *index, int64_t n, int shift,
                         unsigned long long *bad, void *ws, cudaStream_t stream) {
   const Layout l = layout(n, ncounts);
   char *p = static_cast<char *>(ws);
   uint32_t *words = reinterpret_cast<uint32_t *>(p);
   uint16_t *starts = reinterpret_cast<uint16_t *>(p + l.starts), *off16 = reinterpret_cast<uint16_t *>(p + l.off16);
-  BALE_CUDA_OK(cudaMemsetAsync(words, 0, l.words_bytes, stream));
-  auto part = shift == 16 ? bucket_partition_kernel<16> : bucket_partition_kernel<0>;
-  const int psmem = kChunk * 2 + (l.bk.n + 2) * 4;
-  BALE_CUDA_OK(cudaFuncSetAttribute(part, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem));
-  part<<<static_cast<unsigned>(l.nchunks), kPartThreads, psmem, stream>>>(index, n, static_cast<uint64_t>(ncounts),
-                                                                         l.bk, off16, starts, words, bad);
-  BALE_CUDA_OK(cudaGetLastError());
-  const int csmem = static_cast<int>((l.bk.size + 3) / 4 * 16 + l.bk.n * 2);
-  BALE_CUDA_OK(cudaFuncSetAttribute(bucket_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, csmem));
-  const int64_t slots = walk_slots();
-  bucket_count_kernel<<<static_cast<unsigned>(slots), kCountThreads, csmem, stream>>>(
-      off16, starts, l.nchunks, l.bk, part_scale(n, l.bk, slots), counts, static_cast<uint64_t>(ncounts), words);
-  BALE_CUDA_OK(cudaGetLastError());
-  return BALE_OK;
+  return shift == 16 ? launch<16>(counts, ncounts, index, n, nullptr, 0, bad, l, words, starts, off16, stream)
+                     : launch<0>(counts, ncounts, index, n, nullptr, 0, bad, l, words, starts, off16, stream);
+}
+
+bool degrees_bucket_supported(int64_t most, int64_t n) {
+  if (most < 1 || !bucket_supported(2 * most, n)) return false;
+  return layout(2 * most, n).total <= static_cast<size_t>(most) * 8;
+}
+
+int launch_degrees_bucket(uint32_t *deg, int64_t n, const uint64_t *keys, const unsigned *nkeys, int64_t most, int S,
+                          void *ws, cudaStream_t stream) {
+  const Layout l = layout(2 * most, n);
+  char *p = static_cast<char *>(ws);
+  return launch<kEdges>(deg, n, reinterpret_cast<const int64_t *>(keys), 2 * most, nkeys, S, nullptr, l,
+                        reinterpret_cast<uint32_t *>(p), reinterpret_cast<uint16_t *>(p + l.starts),
+                        reinterpret_cast<uint16_t *>(p + l.off16), stream);
 }
 
 }  // namespace bale

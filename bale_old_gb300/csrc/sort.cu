@@ -551,14 +551,14 @@ void launch_csr_check(const int64_t *off, const int64_t *col, int64_t numrows, i
   csr_check_kernel<<<grid_for(std::max(numrows + 1, nnz)), 256, 0, st>>>(off, col, numrows, numcols, nnz, bad);
 }
 
-uint64_t *radix_sort(uint64_t *a, uint64_t *b, int64_t n, int bits, Ws &w, cudaStream_t st, int *rc) {
+uint64_t *radix_sort(uint64_t *a, uint64_t *b, int64_t n, int bits, Ws &w, cudaStream_t st, int *rc, int from) {
   *rc = BALE_OK;
   if (n <= 1) return a;
   if (single_sweep(n)) {
-    *rc = single_sweep_sort(&a, &b, n, 0, (bits + kDigitBits - 1) / kDigitBits, w, st);
+    *rc = single_sweep_sort(&a, &b, n, from, (bits - from + kDigitBits - 1) / kDigitBits, w, st);
     return a;
   }
-  for (int shift = 0; shift < bits; shift += kDigitBits) {
+  for (int shift = from; shift < bits; shift += kDigitBits) {
     *rc = radix_pass_scanned(a, b, n, shift, w, st);
     if (*rc != BALE_OK) return a;
     std::swap(a, b);

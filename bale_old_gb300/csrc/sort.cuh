@@ -28,7 +28,7 @@ struct Ws {
   uint64_t *ka, *kb, *va, *vb;
   uint32_t *flag, *pos, *hist, *hoff, *bsum, *deg, *newid;
   uint32_t *osw;        // kOsWords: the single-sweep sort's digit starts and tile counters
-  unsigned int *words;  // [0] scan total, [1] max degree, [kSortErrWord] a sort wait gave up
+  unsigned int *words;  // [0] scan total, [1] max degree, [2], [3] unique_edges, [kSortErrWord] a sort wait gave up
 };
 
 size_t up256(size_t x);
@@ -55,7 +55,13 @@ int csr_from_keys(const uint64_t *sk, int64_t nk, int64_t nrows, int S, int64_t 
 // [0, numcols).  Asynchronous.
 void launch_csr_check(const int64_t *off, const int64_t *col, int64_t numrows, int64_t numcols, int64_t nnz,
                       unsigned long long *bad, cudaStream_t st);
-// Stable sort of n keys on bits [0, bits); returns the buffer holding the result.
-uint64_t *radix_sort(uint64_t *a, uint64_t *b, int64_t n, int bits, Ws &w, cudaStream_t st, int *rc);
+// Stable sort of n keys on bits [from, bits); returns the buffer holding the result.
+uint64_t *radix_sort(uint64_t *a, uint64_t *b, int64_t n, int bits, Ws &w, cudaStream_t st, int *rc, int from = 0);
 
+// The distinct keys of the m edge keys in w.ka (all-ones: no edge), in any
+// order, into w.ka, and the degrees of their endpoints into w.deg.  words (four,
+// zero before): [0] their number, [2] set when a bucket of the hash did not
+// hold -- then w.kb has the keys of all edges, [3] of them, and the rest is void.
+bool unique_edges_supported(int64_t m, int64_t n);
+int unique_edges(Ws &w, int64_t m, int64_t n, int S, unsigned int *words, cudaStream_t st);
 }  // namespace bale

@@ -15,8 +15,14 @@
 //
 // Here "j's owner" is a CTA or a warp, and the incoming wedges of each j are
 // grouped through the transpose of L, built on the device:
-//   1. scan: validate every row (offsets inside [0,nnz], columns ascending in
-//      [0,i)), write the u32 column copy, count each j's incoming (i, p > 0);
+//   1. rows, scan: validate every row (offsets inside [0,nnz], columns
+//      ascending in [0,i)), write the u32 column copy, count each j's incoming
+//      (i, p > 0).  The scan and the fill split the nonzeros, not the rows,
+//      into equal chunks: a warp's share of a graph with hubs by rows (32 of
+//      them at a time) ran up to 470 rounds of loads against 72 on average,
+//      and a graph of 2^14 rows gave 32 blocks work (R-MAT scale 22: fill
+//      1515 -> 1077 us, scan 449 -> 375; 2^14 rows, 2^18 edges: fill
+//      77 -> 21 us, scan 41 -> 21);
 //   2. exclusive scan of the counts -> in_off;
 //   3. fill: in_rec[in_off[j] + t] = {k - p, p}, the start and length of the
 //      prefix row_i[0,p) (k is the nonzero's index);
@@ -48,8 +54,10 @@ namespace {
 using tri::kBadCol;
 using tri::kFull;
 
-constexpr int kScanThreads = 256;
+constexpr int kScanThreads = 512;
 constexpr int kScanWarps = kScanThreads / 32;
+constexpr int kRowsThreads = 256;
+constexpr int kRowsBlocksPerSm = 8;
 constexpr int kPsumThreads = 1024;
 constexpr int kPsumPer = 4;
 constexpr int64_t kPsumBlock = static_cast<int64_t>(kPsumThreads) * kPsumPer;  // counts per scan block
@@ -57,10 +65,12 @@ constexpr int kWarpThreads = 256;
 constexpr int kWarpWarps = kWarpThreads / 32;
 constexpr int kWarpBitsMax = 16;  // bitmap of 2^16 labels (8 KiB) per warp
 constexpr int kOvf = 256;         // columns at or above 2^16 a warp keeps in shared memory
-constexpr int kUnroll = 4;        // rounds of 32 nonzeros in flight per warp (scan, fill)
+constexpr int kUnroll = 2;        // the scan's rounds of 32 nonzeros in flight per warp (4 spill: 510 against 375 us)
 constexpr int kHub = 8192;        // labels whose incoming counts and slots live in shared memory
-constexpr int kScanBlocksPerSm = 6;
-constexpr int kFillUnroll = 4;     // the fill's rounds in flight
+constexpr int kScanBlocksPerSm = 3;
+constexpr uint32_t kChunkMin = 256;     // nonzeros of a chunk at least: two rounds of the fill
+constexpr uint32_t kChunksPerWarp = 4;  // chunks a warp takes in turn when the scan fills the GPU
+constexpr int kFillUnroll = 4;     // the fill's rounds in flight (chunks are a multiple of them)
 constexpr int kProbeInFlight = 5;  // 16-byte prefix vectors per lane in flight when probing
 constexpr int kStagedInFlight = 2; // the same for prefixes probed against staged short rows
 constexpr int kDenseHubs = 16384;  // rows j below this keep a bitmap of their columns for dense pairs
@@ -68,8 +78,9 @@ constexpr int kDenseThreads = 256;
 
 // Workspace words: [0] nonzero when the scan met a dense pair, [1] malformed
 // entries seen by the scan, [2] the dense-pair margin (negative: no dense
-// pairs), [3] the bitmap rows (a multiple of 128).
-enum { kWDenseAny = 0, kWBad = 1, kWDenseOv = 2, kWDenseHubs = 3, kWords = 4 };
+// pairs), [3] the bitmap rows (a multiple of 128), [4] rows with offsets
+// outside [0,nnz] or descending (also counted in [1]).
+enum { kWDenseAny = 0, kWBad = 1, kWDenseOv = 2, kWDenseHubs = 3, kWBadRows = 4, kWords = 8 };
 
 // A nonzero (i, j) at position p of row i is a dense pair when j has a
 // column bitmap (j < hubs) and its prefix row_i[0,p) is longer than the
@@ -81,8 +92,11 @@ __device__ __forceinline__ bool dense_pair(uint32_t j, uint32_t p, int64_t ov, u
 }
 
 struct Layout {
-  size_t col32, in_cnt, in_off, bsum, in_rec, hubs, bits, words, total;
+  size_t col32, in_cnt, in_off, bsum, in_rec, hubs, bits, starts, words, total;
   uint32_t dense_hubs;  // rows with a column bitmap: min(kDenseHubs, numrows rounded up to 128)
+  uint32_t chunk;       // nonzeros per chunk of the scan and the fill (a multiple of a warp's round)
+  uint32_t nchunks;
+  uint32_t blocks;      // blocks of the scan and the fill
 };
 
 size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -97,10 +111,19 @@ Layout layout(int64_t n, int64_t nnz) {
   l.in_off = o; o += up256(static_cast<size_t>(n + 1) * 4);
   l.bsum = o;   o += up256(nb * 4);
   l.in_rec = o; o += up256(nz * 8);
-  l.hubs = o;   o += up256(static_cast<size_t>(num_sms()) * kScanBlocksPerSm * kHub * 4);
+  // chunks of equal length, one a warp until every warp of the GPU has
+  // kChunksPerWarp of them, longer ones beyond that
+  const size_t warps = static_cast<size_t>(num_sms()) * kScanBlocksPerSm * kScanWarps;
+  const size_t want = (nz + warps * kChunksPerWarp - 1) / (warps * kChunksPerWarp);
+  l.chunk = static_cast<uint32_t>(std::max<size_t>(kChunkMin, (want + 32 * kFillUnroll - 1) / (32 * kFillUnroll) * (32 * kFillUnroll)));
+  l.nchunks = static_cast<uint32_t>((nz + l.chunk - 1) / l.chunk);
+  l.blocks = static_cast<uint32_t>(std::min<size_t>((l.nchunks + kScanWarps - 1) / kScanWarps,
+                                                    static_cast<size_t>(num_sms()) * kScanBlocksPerSm));
+  l.hubs = o;   o += up256(static_cast<size_t>(l.blocks) * kHub * 4);
   // a multiple of 128, so each row's bitmap starts on a 16-byte boundary
   l.dense_hubs = static_cast<uint32_t>(std::min<int64_t>(kDenseHubs, (n + 127) / 128 * 128));
   l.bits = o;   o += up256(static_cast<size_t>(l.dense_hubs) * (l.dense_hubs / 32) * 4);
+  l.starts = o; o += up256(static_cast<size_t>(l.nchunks) * 4);
   l.words = o;  o += up256(kWords * 8);
   l.total = o;
   return l;
@@ -141,139 +164,278 @@ __device__ __forceinline__ int flat_owner(uint32_t inc, uint32_t bb) {
   return o < 32u ? static_cast<int>(o) : 31;
 }
 
-// The nonzeros of 32 consecutive rows, flattened over the warp.  The rows'
-// offsets are loaded one per lane; rows whose offsets are not inside
-// [0,nnz] count as bad.  The non-empty rows are compacted to the low lanes
-// through the warp's 32-entry staging slot so that their prefixes strictly
-// increase (flat_owner's condition).
-struct RowGroup {
-  uint32_t b = 0, d = 0, row = 0, inc = 0, tot = 0;
-  unsigned nbad = 0;
-  __device__ __forceinline__ void load(const int64_t *__restrict__ off, int64_t n, int64_t nnz, int64_t r0,
-                                       uint4 *slot) {
-    const unsigned lane = lane_id();
-    const int64_t i = r0 + lane;
-    uint32_t mb = 0, md = 0;
-    if (i < n) {
-      const int64_t bb = off[i], e = off[i + 1];
-      if (bb < 0 || e < bb || e > nnz) {
-        nbad = 1;
-      } else {
-        mb = static_cast<uint32_t>(bb);
-        md = static_cast<uint32_t>(e - bb);
-      }
+// Row offsets: rows outside [0,nnz] or descending are counted (the later
+// kernels then return before they use any), the incoming counts are zeroed,
+// and starts[c] becomes the row that holds nonzero c * chunk -- so the scan
+// and the fill can split the nonzeros evenly, whatever the rows' lengths.
+// Chunks before the first row's start begin at row 0, those past the last
+// row's end at row n (no rows).
+__global__ void __launch_bounds__(kRowsThreads)
+    wedge_rows_kernel(const int64_t *__restrict__ off, int64_t n, int64_t nnz, uint32_t *__restrict__ in_cnt,
+                      uint32_t *__restrict__ starts, uint32_t chunk, uint32_t nchunks,
+                      unsigned long long *__restrict__ words, unsigned long long *__restrict__ bad,
+                      const unsigned *__restrict__ run_if) {
+  if (tri::skipped(run_if, 1u)) return;
+  unsigned long long nbad = 0;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * kRowsThreads;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * kRowsThreads + threadIdx.x; i < n; i += stride) {
+    in_cnt[i] = 0;
+    const int64_t b = off[i], e = off[i + 1];
+    if (b < 0 || e < b || e > nnz) {
+      nbad++;
+      continue;
     }
-    const unsigned m = __ballot_sync(kFull, md > 0);
-    if (md > 0) slot[__popc(m & ((1u << lane) - 1u))] = make_uint4(mb, md, lane, 0u);
+    // nnz < 2^32 - 256, so offsets and chunk starts fit 32 bits
+    const uint32_t b32 = static_cast<uint32_t>(b), e32 = static_cast<uint32_t>(e);
+    uint32_t c = b32 / chunk + (b32 % chunk ? 1u : 0u);
+    if (i == 0)
+      for (uint32_t t = 0; t < c && t < nchunks; t++) starts[t] = 0;
+    for (; c < nchunks && c * chunk < e32; c++) starts[c] = static_cast<uint32_t>(i);
+    if (i == n - 1)
+      for (; c < nchunks; c++) starts[c] = static_cast<uint32_t>(n);
+  }
+  nbad = warp_sum_u64(nbad);
+  if (lane_id() == 0 && nbad) {
+    atomicAdd(words + kWBad, nbad);
+    atomicAdd(words + kWBadRows, nbad);
+    if (bad) atomicAdd(bad, nbad);
+  }
+}
+
+// The nonzeros [k0,k1) (a chunk) that lie in 32 consecutive rows, flattened
+// over the warp.  The rows' offsets (ascending and inside [0,nnz]) are one
+// per lane; the rows with nonzeros in the chunk are compacted to the low
+// lanes through the warp's 32-entry staging slot so that their prefixes
+// strictly increase (flat_owner's condition).
+struct RowWindow {
+  uint32_t first = 0, b = 0, row = 0, inc = 0, tot = 0;
+  __device__ __forceinline__ void set(uint32_t mb, uint32_t me, uint32_t k0, uint32_t k1, uint4 *slot) {
+    const unsigned lane = lane_id();
+    const uint32_t lo = mb > k0 ? mb : k0, hi = me < k1 ? me : k1;
+    const bool live = hi > lo;
+    const unsigned m = __ballot_sync(kFull, live);
+    if (live) slot[__popc(m & ((1u << lane) - 1u))] = make_uint4(lo, hi - lo, lane, mb);
     __syncwarp();
+    uint32_t d = 0;
     if (lane < static_cast<unsigned>(__popc(m))) {
       const uint4 t = slot[lane];
-      b = t.x;
+      first = t.x;
       d = t.y;
       row = t.z;
+      b = t.w;
     }
     __syncwarp();
     inc = incl_scan_u32(d);
+    first -= inc - d;  // nonzero index = first + flattened position
     tot = __shfl_sync(kFull, inc, 31);
   }
   // Nonzero index k, its position p in its row and the row (relative to the
-  // group) of flattened position bb + lane (all lanes call; valid for < tot).
+  // window) of flattened position bb + lane (all lanes call; valid for < tot).
   __device__ __forceinline__ void at(uint32_t bb, uint32_t &k, uint32_t &p, uint32_t &r) const {
     const int o = flat_owner(inc, bb);
-    const uint32_t ob = __shfl_sync(kFull, b, o);
-    const uint32_t ox = __shfl_sync(kFull, inc - d, o);
+    k = __shfl_sync(kFull, first, o) + bb + lane_id();
+    p = k - __shfl_sync(kFull, b, o);
     r = __shfl_sync(kFull, row, o);
-    p = bb + lane_id() - ox;
-    k = ob + p;
   }
 };
+
+// The row r of [lo,n) with off[r] <= k < off[r + 1], for ascending offsets
+// with off[lo] <= k < off[n] (whole warp; 32 places tested per step).
+__device__ __forceinline__ int64_t row_of(const int64_t *__restrict__ off, int64_t lo, int64_t n, int64_t k) {
+  int64_t hi = n;
+  while (hi - lo > 1) {
+    const int64_t step = (hi - lo + 31) / 32;
+    const int64_t at = lo + (static_cast<int64_t>(lane_id()) + 1) * step;
+    const int64_t c = __popc(__ballot_sync(kFull, at < hi && off[at] <= k));
+    const int64_t up = lo + (c + 1) * step;
+    lo += c * step;
+    hi = up < hi ? up : hi;
+  }
+  return lo;
+}
+
+// Calls f(window, first row) for each window of 32 rows that holds nonzeros
+// of the chunk [k0,k1), which begins in row r0.  The next window's offsets
+// are loaded before f runs.  A stretch of empty rows is crossed by a search.
+template <class F>
+__device__ __forceinline__ void for_windows(const int64_t *__restrict__ off, int64_t n, int64_t r0, uint32_t k0,
+                                            uint32_t k1, uint4 *slot, F f) {
+  const int64_t lane = static_cast<int64_t>(lane_id());
+  uint32_t b = 0, e = 0;
+  if (r0 + lane < n) {
+    b = static_cast<uint32_t>(off[r0 + lane]);
+    e = static_cast<uint32_t>(off[r0 + lane + 1]);
+  }
+  while (r0 < n) {
+    // off[min(r0 + 32, n)], where the next window begins
+    const uint32_t end = __reduce_max_sync(kFull, e);
+    const bool last = r0 + 32 >= n || end >= k1;
+    uint32_t nb = 0, ne = 0;
+    if (!last && r0 + 32 + lane < n) {
+      nb = static_cast<uint32_t>(off[r0 + 32 + lane]);
+      ne = static_cast<uint32_t>(off[r0 + 32 + lane + 1]);
+    }
+    RowWindow w;
+    w.set(b, e, k0, k1, slot);
+    if (w.tot) f(w, r0);
+    if (last) return;
+    r0 += 32;
+    b = nb;
+    e = ne;
+    if (__reduce_max_sync(kFull, e) <= end && r0 + 32 < n) {  // an empty window
+      if (static_cast<int64_t>(end) >= off[n]) return;
+      r0 = row_of(off, r0, n, end);
+      b = e = 0;
+      if (r0 + lane < n) {
+        b = static_cast<uint32_t>(off[r0 + lane]);
+        e = static_cast<uint32_t>(off[r0 + lane + 1]);
+      }
+    }
+  }
+}
+
+// *a += 1 in shared memory where `on` holds; the form with a result gives
+// the old value (0 elsewhere).  Predicated: a branch around each costs more
+// than the atomic.
+__device__ __forceinline__ void count_shared(uint32_t *a, bool on) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %1, 0;\n @q red.shared.add.u32 [%0], 1;\n}" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(a))),
+               "r"(static_cast<uint32_t>(on))
+               : "memory");
+}
+
+__device__ __forceinline__ uint32_t take_shared(uint32_t *a, bool on) {
+  uint32_t v = 0;
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q atom.shared.add.u32 %0, [%1], 1;\n}"
+               : "+r"(v)
+               : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(a))), "r"(static_cast<uint32_t>(on))
+               : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void count_global(uint32_t *a, bool on) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %1, 0;\n @q red.global.add.u32 [%0], 1;\n}" ::"l"(a),
+               "r"(static_cast<uint32_t>(on))
+               : "memory");
+}
+
+__device__ __forceinline__ uint32_t take_global(uint32_t *a, bool on) {
+  uint32_t v = 0;
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q atom.global.add.u32 %0, [%1], 1;\n}"
+               : "+r"(v)
+               : "l"(a), "r"(static_cast<uint32_t>(on))
+               : "memory");
+  return v;
+}
 
 // Incoming counts of hub labels (below kHub) are accumulated per block in
 // shared memory: on a degree-ordered matrix nearly every row starts with
 // the same few hubs, and their global counters would serialise in L2.  Each
-// block's hub counts go to hubs[block][label] (for the fill's slot bases)
-// and into in_cnt once.
-__global__ void __launch_bounds__(kScanThreads)
+// block's hub counts go to hubs[block][label], from which the hub scan makes
+// the fill's slot bases and the labels' counts.
+__global__ void __launch_bounds__(kScanThreads, kScanBlocksPerSm)
     wedge_scan_kernel(const int64_t *__restrict__ off, const int64_t *__restrict__ col, int64_t n, int64_t nnz,
+                      const uint32_t *__restrict__ starts, uint32_t chunk, uint32_t nchunks,
                       uint32_t *__restrict__ col32, uint32_t *__restrict__ in_cnt, uint32_t *__restrict__ hubs,
                       unsigned long long *__restrict__ words, unsigned long long *__restrict__ bad, int64_t ov,
                       uint32_t dhubs, const unsigned *__restrict__ run_if) {
   if (tri::skipped(run_if, 1u)) return;
+  if (words[kWBadRows]) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     words[kWDenseOv] = static_cast<unsigned long long>(ov);
     words[kWDenseHubs] = dhubs;
   }
   __shared__ uint4 stage[kScanWarps][32];
   __shared__ uint32_t hub[kHub];
-  for (int h = threadIdx.x; h < kHub; h += kScanThreads) hub[h] = 0;
+  const int hlim = n < kHub ? static_cast<int>(n) : kHub;
+  for (int h = threadIdx.x; h < hlim; h += kScanThreads) hub[h] = 0;
   __syncthreads();
-  const int64_t groups = (n + 31) / 32;
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * kScanWarps;
+  const uint32_t warps = gridDim.x * kScanWarps;
   const unsigned lane = lane_id();
-  unsigned long long nbad = 0;
+  unsigned nbad = 0;
   bool any_dense = false;
-  for (int64_t g = static_cast<int64_t>(blockIdx.x) * kScanWarps + (threadIdx.x >> 5); g < groups; g += warps) {
-    RowGroup rg;
-    rg.load(off, n, nnz, g * 32, stage[threadIdx.x >> 5]);
-    nbad += rg.nbad;
-    uint32_t carry = 0;  // the element before this batch (lane 31 of the last round)
-    for (uint32_t base = 0; base < rg.tot; base += 32 * kUnroll) {
-      uint32_t k[kUnroll], p[kUnroll], r[kUnroll], cu[kUnroll];
-      int64_t c[kUnroll];
+  for (uint32_t c = blockIdx.x * kScanWarps + (threadIdx.x >> 5); c < nchunks; c += warps) {
+    const uint32_t k0 = c * chunk;
+    const uint32_t k1 = static_cast<uint32_t>(nnz) - k0 < chunk ? static_cast<uint32_t>(nnz) : k0 + chunk;
+    // the element before this round's first (lane 31 of the last round, or of the chunk before)
+    const int64_t before = k0 > 0 ? col[k0 - 1] : 0;
+    uint32_t carry = (before >= 0 && before < static_cast<int64_t>(kBadCol)) ? static_cast<uint32_t>(before) : kBadCol;
+    for_windows(off, n, starts[c], k0, k1, stage[threadIdx.x >> 5], [&](const RowWindow &w, int64_t r0) {
+      for (uint32_t base = 0; base < w.tot; base += 32 * kUnroll) {
+        uint32_t k[kUnroll], p[kUnroll], r[kUnroll], cu[kUnroll];
+        int64_t cv[kUnroll];
 #pragma unroll
-      for (int u = 0; u < kUnroll; u++) {
-        rg.at(base + 32 * u, k[u], p[u], r[u]);
-        c[u] = base + 32 * u + lane < rg.tot ? ld_stream(col + k[u]) : 0;
-        cu[u] = (c[u] >= 0 && c[u] < static_cast<int64_t>(kBadCol)) ? static_cast<uint32_t>(c[u]) : kBadCol;
-      }
-#pragma unroll
-      for (int u = 0; u < kUnroll; u++) {
-        // the previous element of the same row: lane - 1 of this round, or
-        // lane 31 of the previous one (flattened positions are consecutive)
-        uint32_t prv = __shfl_up_sync(kFull, cu[u], 1);
-        const uint32_t last = __shfl_sync(kFull, u == 0 ? carry : cu[u > 0 ? u - 1 : 0], 31);
-        if (lane == 0) prv = last;
-        if (base + 32 * u + lane < rg.tot) {
-          const int64_t i = g * 32 + r[u];
-          const bool ok = c[u] >= 0 && c[u] < i && (p[u] == 0 || cu[u] > prv);
-          col32[k[u]] = ok ? cu[u] : kBadCol;
-          if (!ok) nbad++;
-          else if (p[u] > 0 && dense_pair(cu[u], p[u], ov, dhubs)) {
-            any_dense = true;
-          } else if (p[u] > 0) {
-            if (cu[u] < static_cast<uint32_t>(kHub)) atomicAdd(&hub[cu[u]], 1u);
-            else atomicAdd(in_cnt + cu[u], 1u);
-          }
+        for (int u = 0; u < kUnroll; u++) {
+          w.at(base + 32 * u, k[u], p[u], r[u]);
+          cv[u] = base + 32 * u + lane < w.tot ? ld_stream(col + k[u]) : 0;
+          cu[u] = (cv[u] >= 0 && cv[u] < static_cast<int64_t>(kBadCol)) ? static_cast<uint32_t>(cv[u]) : kBadCol;
         }
+#pragma unroll
+        for (int u = 0; u < kUnroll; u++) {
+          // the previous element of the same row: lane - 1 of this round, or
+          // lane 31 of the previous one (flattened positions are consecutive)
+          uint32_t prv = __shfl_up_sync(kFull, cu[u], 1);
+          const uint32_t end = __shfl_sync(kFull, u == 0 ? carry : cu[u > 0 ? u - 1 : 0], 31);
+          if (lane == 0) prv = end;
+          const bool in = base + 32 * u + lane < w.tot;
+          const bool ok = cu[u] < static_cast<uint32_t>(r0) + r[u] && (p[u] == 0 || cu[u] > prv);
+          if (in) col32[k[u]] = ok ? cu[u] : kBadCol;
+          nbad += in && !ok;
+          const bool inner = in && ok && p[u] > 0;
+          const bool dense = inner && dense_pair(cu[u], p[u], ov, dhubs);
+          any_dense |= dense;
+          count_shared(&hub[cu[u] & (kHub - 1)], inner && !dense && cu[u] < static_cast<uint32_t>(kHub));
+          count_global(in_cnt + cu[u], inner && !dense && cu[u] >= static_cast<uint32_t>(kHub));
+        }
+        carry = cu[kUnroll - 1];
       }
-      carry = cu[kUnroll - 1];
-    }
+    });
   }
-  nbad = warp_sum_u64(nbad);
+  nbad = __reduce_add_sync(kFull, nbad);
   if (lane == 0 && nbad) {
-    atomicAdd(words + kWBad, nbad);
-    if (bad) atomicAdd(bad, nbad);
+    atomicAdd(words + kWBad, static_cast<unsigned long long>(nbad));
+    if (bad) atomicAdd(bad, static_cast<unsigned long long>(nbad));
   }
   if (__syncthreads_or(any_dense) && threadIdx.x == 0) words[kWDenseAny] = 1;
   uint32_t *mine = hubs + static_cast<size_t>(blockIdx.x) * kHub;
-  for (int h = threadIdx.x; h < kHub; h += kScanThreads) {
-    const uint32_t v = hub[h];
-    mine[h] = v;
-    if (v) atomicAdd(in_cnt + h, v);
-  }
+  for (int h = threadIdx.x; h < hlim; h += kScanThreads) mine[h] = hub[h];
 }
 
-// hubs[b][h] becomes the exclusive prefix over blocks b of the hub counts.
-__global__ void __launch_bounds__(256) wedge_hubscan_kernel(uint32_t *__restrict__ hubs, int nblocks, const unsigned *__restrict__ run_if) {
+// hubs[b][h] becomes the exclusive prefix over blocks b of the hub counts,
+// in_cnt[h] their sum.  A block takes 32 labels, its 32 warps each a run of
+// the scan's blocks, whose loads do not wait on one another (one thread per
+// label took 71 us for 912 blocks).
+__global__ void __launch_bounds__(1024)
+    wedge_hubscan_kernel(uint32_t *__restrict__ hubs, int nblocks, int hlim, uint32_t *__restrict__ in_cnt,
+                         const unsigned *__restrict__ run_if) {
   if (tri::skipped(run_if, 1u)) return;
-  const int h = blockIdx.x * 256 + threadIdx.x;
-  if (h >= kHub) return;
-  uint32_t run = 0;
-  for (int b = 0; b < nblocks; b++) {
+  __shared__ uint32_t sums[32][33];
+  const unsigned lane = lane_id(), y = threadIdx.x >> 5;
+  const int h = blockIdx.x * 32 + lane;
+  const int per = (nblocks + 31) / 32;
+  const int b0 = static_cast<int>(y) * per, b1 = b0 + per < nblocks ? b0 + per : nblocks;
+  uint32_t sum = 0;
+  if (h < hlim) {
+#pragma unroll 8
+    for (int b = b0; b < b1; b++) sum += hubs[static_cast<size_t>(b) * kHub + h];
+  }
+  sums[y][lane] = sum;
+  __syncthreads();
+  // warp y scans label y's 32 runs
+  const uint32_t v = sums[lane][y];
+  const uint32_t inc = incl_scan_u32(v);
+  __syncwarp();
+  sums[lane][y] = inc - v;
+  if (lane == 31 && blockIdx.x * 32 + y < static_cast<unsigned>(hlim)) in_cnt[blockIdx.x * 32 + y] = inc;
+  __syncthreads();
+  if (h >= hlim) return;
+  uint32_t run = sums[y][lane];
+#pragma unroll 8
+  for (int b = b0; b < b1; b++) {
     uint32_t *x = hubs + static_cast<size_t>(b) * kHub + h;
-    const uint32_t v = *x;
+    const uint32_t t = *x;
     *x = run;
-    run += v;
+    run += t;
   }
 }
 
@@ -334,7 +496,8 @@ __global__ void __launch_bounds__(kPsumThreads)
   if (threadIdx.x == 0) in_off[n] = carry;
 }
 
-// in_off[j] = exclusive prefix of the counts; the counts are zeroed for the fill.
+// in_off[j] = exclusive prefix of the counts; the counts become the fill's
+// next slot of each j.
 __global__ void __launch_bounds__(kPsumThreads)
     wedge_offsets_kernel(uint32_t *__restrict__ in_cnt, int64_t n, const uint32_t *__restrict__ bsum,
                          uint32_t *__restrict__ in_off, const unsigned *__restrict__ run_if) {
@@ -348,17 +511,18 @@ __global__ void __launch_bounds__(kPsumThreads)
   for (int q = 0; q < 4; q++) {
     if (idx + q < n) {
       in_off[idx + q] = x;
-      in_cnt[idx + q] = 0;
+      in_cnt[idx + q] = x;
     }
     x += v[q];
   }
 }
 
-// Same grid and the same rows per block as the scan, so a block's hub
+// Same grid and the same chunks per block as the scan, so a block's hub
 // records take the slots in_off[h] + hubs[block][h] onwards, handed out by
 // shared-memory counters; other labels take global ones.
-__global__ void __launch_bounds__(kScanThreads)
+__global__ void __launch_bounds__(kScanThreads, kScanBlocksPerSm)
     wedge_fill_kernel(const int64_t *__restrict__ off, const uint32_t *__restrict__ col32, int64_t n, int64_t nnz,
+                      const uint32_t *__restrict__ starts, uint32_t chunk, uint32_t nchunks,
                       const uint32_t *__restrict__ in_off, uint32_t *__restrict__ in_cnt,
                       const uint32_t *__restrict__ hubs, uint2 *__restrict__ in_rec,
                       const unsigned long long *__restrict__ words, const unsigned *__restrict__ run_if) {
@@ -368,36 +532,39 @@ __global__ void __launch_bounds__(kScanThreads)
   if (words[kWBad]) return;
   const int64_t ov = static_cast<int64_t>(words[kWDenseOv]);
   const uint32_t dhubs = static_cast<uint32_t>(words[kWDenseHubs]);
+  const int hlim = n < kHub ? static_cast<int>(n) : kHub;
   {
     const uint32_t *mine = hubs + static_cast<size_t>(blockIdx.x) * kHub;
-    for (int h = threadIdx.x; h < kHub; h += kScanThreads) hubslot[h] = h < n ? in_off[h] + mine[h] : 0u;
+    for (int h = threadIdx.x; h < hlim; h += kScanThreads) hubslot[h] = in_off[h] + mine[h];
     __syncthreads();
   }
-  const int64_t groups = (n + 31) / 32;
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * kScanWarps;
+  const uint32_t warps = gridDim.x * kScanWarps;
   const unsigned lane = lane_id();
-  for (int64_t g = static_cast<int64_t>(blockIdx.x) * kScanWarps + (threadIdx.x >> 5); g < groups; g += warps) {
-    RowGroup rg;
-    rg.load(off, n, nnz, g * 32, stage[threadIdx.x >> 5]);
-    for (uint32_t base = 0; base < rg.tot; base += 32 * kFillUnroll) {
-      uint32_t k[kFillUnroll], p[kFillUnroll], c[kFillUnroll], slot[kFillUnroll];
+  for (uint32_t ch = blockIdx.x * kScanWarps + (threadIdx.x >> 5); ch < nchunks; ch += warps) {
+    const uint32_t k0 = ch * chunk;
+    const uint32_t k1 = static_cast<uint32_t>(nnz) - k0 < chunk ? static_cast<uint32_t>(nnz) : k0 + chunk;
+    for_windows(off, n, starts[ch], k0, k1, stage[threadIdx.x >> 5], [&](const RowWindow &w, int64_t) {
+      for (uint32_t base = 0; base < w.tot; base += 32 * kFillUnroll) {
+        uint32_t k[kFillUnroll], p[kFillUnroll], c[kFillUnroll], slot[kFillUnroll];
 #pragma unroll
-      for (int u = 0; u < kFillUnroll; u++) {
-        uint32_t r;
-        rg.at(base + 32 * u, k[u], p[u], r);
-        c[u] = base + 32 * u + lane < rg.tot ? col32[k[u]] : kBadCol;
-        // the first nonzero of a row closes no wedge; dense pairs are counted apart
-        if (p[u] == 0 || (c[u] != kBadCol && dense_pair(c[u], p[u], ov, dhubs))) c[u] = kBadCol;
+        for (int u = 0; u < kFillUnroll; u++) {
+          uint32_t r;
+          w.at(base + 32 * u, k[u], p[u], r);
+          c[u] = base + 32 * u + lane < w.tot ? col32[k[u]] : kBadCol;
+          // the first nonzero of a row closes no wedge; dense pairs are counted apart
+          if (p[u] == 0 || (c[u] != kBadCol && dense_pair(c[u], p[u], ov, dhubs))) c[u] = kBadCol;
+        }
+#pragma unroll
+        for (int u = 0; u < kFillUnroll; u++) {
+          const uint32_t s = take_shared(&hubslot[c[u] & (kHub - 1)], c[u] < static_cast<uint32_t>(kHub));
+          const uint32_t g = take_global(in_cnt + c[u], c[u] >= static_cast<uint32_t>(kHub) && c[u] != kBadCol);
+          slot[u] = s + g;  // one of them is 0
+        }
+#pragma unroll
+        for (int u = 0; u < kFillUnroll; u++)
+          if (c[u] != kBadCol) in_rec[slot[u]] = make_uint2(k[u] - p[u], p[u]);
       }
-#pragma unroll
-      for (int u = 0; u < kFillUnroll; u++)
-        slot[u] = c[u] == kBadCol               ? 0u
-                  : c[u] < static_cast<uint32_t>(kHub) ? atomicAdd(&hubslot[c[u]], 1u)
-                                                : in_off[c[u]] + atomicAdd(in_cnt + c[u], 1u);
-#pragma unroll
-      for (int u = 0; u < kFillUnroll; u++)
-        if (c[u] != kBadCol) in_rec[slot[u]] = make_uint2(k[u] - p[u], p[u]);
-    }
+    });
   }
 }
 
@@ -845,24 +1012,26 @@ int tri_wedge_prepare(const int64_t *offset, const int64_t *nonzero, int64_t num
   uint32_t *hubs = reinterpret_cast<uint32_t *>(p + l.hubs);
   uint32_t *bits = reinterpret_cast<uint32_t *>(p + l.bits);
   unsigned long long *words = reinterpret_cast<unsigned long long *>(p + l.words);
-  const int sms = num_sms();
+  uint32_t *starts = reinterpret_cast<uint32_t *>(p + l.starts);
   // dense pairs (tri.dense 0: none) and their margin over the bitmap's words
   const int64_t ov = knob_or("tri.dense", 1) == 0 ? -1 : knob_or("tri.dense_ov", 32);
-  BALE_CUDA_OK(cudaMemsetAsync(in_cnt, 0, static_cast<size_t>(numrows) * 4, stream));
   BALE_CUDA_OK(cudaMemsetAsync(words, 0, kWords * sizeof(unsigned long long), stream));
-  const int64_t groups = (numrows + 31) / 32;
-  int64_t sblocks = (groups + kScanWarps - 1) / kScanWarps;
-  const int64_t scap = static_cast<int64_t>(sms) * kScanBlocksPerSm;  // the hubs array holds this many blocks
-  if (sblocks > scap) sblocks = scap;
-  wedge_scan_kernel<<<static_cast<unsigned>(sblocks), kScanThreads, 0, stream>>>(
-      offset, nonzero, numrows, nnz, col32, in_cnt, hubs, words, bad, ov, l.dense_hubs, run_if);
+  const int64_t rblocks = std::min<int64_t>((numrows + kRowsThreads - 1) / kRowsThreads,
+                                            static_cast<int64_t>(num_sms()) * kRowsBlocksPerSm);
+  wedge_rows_kernel<<<static_cast<unsigned>(rblocks), kRowsThreads, 0, stream>>>(
+      offset, numrows, nnz, in_cnt, starts, l.chunk, l.nchunks, words, bad, run_if);
+  BALE_CUDA_OK(cudaGetLastError());
+  wedge_scan_kernel<<<l.blocks, kScanThreads, 0, stream>>>(offset, nonzero, numrows, nnz, starts, l.chunk, l.nchunks,
+                                                           col32, in_cnt, hubs, words, bad, ov, l.dense_hubs, run_if);
   BALE_CUDA_OK(cudaGetLastError());
   if (ov >= 0 && l.dense_hubs > 0) {
     wedge_hubbits_kernel<<<static_cast<unsigned>((l.dense_hubs + 7) / 8), 256, 0, stream>>>(offset, col32, numrows,
                                                                                             bits, words, run_if);
     BALE_CUDA_OK(cudaGetLastError());
   }
-  wedge_hubscan_kernel<<<kHub / 256, 256, 0, stream>>>(hubs, static_cast<int>(sblocks), run_if);
+  const int64_t hlim = std::min<int64_t>(kHub, numrows);
+  wedge_hubscan_kernel<<<static_cast<unsigned>((hlim + 31) / 32), 1024, 0, stream>>>(
+      hubs, static_cast<int>(l.blocks), static_cast<int>(hlim), in_cnt, run_if);
   BALE_CUDA_OK(cudaGetLastError());
   const int64_t nb = (numrows + kPsumBlock - 1) / kPsumBlock;
   wedge_blocksum_kernel<<<static_cast<unsigned>(nb), kPsumThreads, 0, stream>>>(in_cnt, numrows, bsum, run_if);
@@ -872,8 +1041,8 @@ int tri_wedge_prepare(const int64_t *offset, const int64_t *nonzero, int64_t num
   wedge_offsets_kernel<<<static_cast<unsigned>(nb), kPsumThreads, 0, stream>>>(in_cnt, numrows, bsum, in_off,
                                                                                run_if);
   BALE_CUDA_OK(cudaGetLastError());
-  wedge_fill_kernel<<<static_cast<unsigned>(sblocks), kScanThreads, 0, stream>>>(offset, col32, numrows, nnz, in_off,
-                                                                                 in_cnt, hubs, in_rec, words, run_if);
+  wedge_fill_kernel<<<l.blocks, kScanThreads, 0, stream>>>(offset, col32, numrows, nnz, starts, l.chunk, l.nchunks,
+                                                           in_off, in_cnt, hubs, in_rec, words, run_if);
   BALE_CUDA_OK(cudaGetLastError());
   return BALE_OK;
 }

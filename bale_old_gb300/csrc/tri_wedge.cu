@@ -24,15 +24,24 @@
 //      1515 -> 1077 us, scan 449 -> 375; 2^14 rows, 2^18 edges: fill
 //      77 -> 21 us, scan 41 -> 21);
 //   2. exclusive scan of the counts -> in_off;
-//   3. fill: in_rec[in_off[j] + t] = {k - p, p}, the start and length of the
-//      prefix row_i[0,p) (k is the nonzero's index);
-//   4. count: one warp per j.  Row j's columns below 2^16 become a bitmap in
-//      the warp's own 8 KiB of shared memory (so no block-wide barrier is
-//      ever needed) and its few columns above 2^16 a short sorted list beside
-//      it; the warp tests every element of the incoming prefixes -- one
-//      shared-memory load per element for the bitmap part -- then clears the
-//      bits it set.  On a degree-ordered matrix the labels below 2^16 are the
-//      hubs, where nearly all probes land (94% at R-MAT scale 22).
+//   3. fill: in_rec[in_off[j] + t] = the prefix row_i[0,p): for near rows j
+//      (below 2^15) where its 16-bit copy starts and p, for the others i and p;
+//   4. count: one warp per j.  Row j's low columns (below 2^15 - 1) become a
+//      bitmap in the warp's own 4 KiB of shared memory (so no block-wide
+//      barrier is ever needed); the warp tests every element of the incoming
+//      prefixes, one shared-memory load each, then clears the bits it set.
+//      Near rows have low columns only, and on a degree-ordered matrix they
+//      are the hubs, where most probes land (80% at R-MAT scale 22); a far
+//      row's other columns are a short sorted list behind a filter.
+//      The prefixes are read from a copy of the rows in 16 bits, each row on
+//      a 16-byte boundary and padded so that whole vectors are probed without
+//      a test of where they end: 8 elements and 75 instructions per vector and
+//      lane instead of 4 and 108, half the bytes.  Warps claim equal shares of
+//      the records, not rows: a hub's 54 K prefixes took one warp 2.3 ms.
+//      R-MAT scale 22: 3980 us with 32-bit rows, a 2^16-bit bitmap per
+//      warp (24 warps an SM) and a claim per row; 2806 with 16-bit rows; 2500
+//      as it is, near (40 warps an SM, its shared-memory data pipe 91% busy)
+//      1330 us and far (32 warps, waiting for dependent loads) 1170.
 //   5. dense pairs: a pair (i,j) whose prefix is longer than the ceil(j/32)
 //      words of a bitmap of [0,j) (plus a margin), for j below 2^14, gets no
 //      record in steps 1-3; step 1 also builds the column bitmaps of the rows
@@ -44,6 +53,7 @@
 // tally is the number of probes, sum_i C(d_i,2) -- the reference's exstack
 // push count -- with each dense pair counted as the p probes it replaces.
 #include <algorithm>
+#include <type_traits>
 
 #include "tri_device.cuh"
 
@@ -63,15 +73,32 @@ constexpr int kPsumPer = 4;
 constexpr int64_t kPsumBlock = static_cast<int64_t>(kPsumThreads) * kPsumPer;  // counts per scan block
 constexpr int kWarpThreads = 256;
 constexpr int kWarpWarps = kWarpThreads / 32;
-constexpr int kWarpBitsMax = 16;  // bitmap of 2^16 labels (8 KiB) per warp
-constexpr int kOvf = 256;         // columns at or above 2^16 a warp keeps in shared memory
+constexpr int kNearBits = 15;
+constexpr uint32_t kNear = 1u << kNearBits;  // rows j below it are near: all their columns are low
+constexpr uint32_t kLow = kNear - 1;         // labels below it are low: bits of a bitmap, values of rows16
+constexpr int kTail = 128;                   // columns of a far row that are not low in shared memory
+constexpr int kFilterWords = 128;            // bits of the filter of those columns, in words
+constexpr int kFarWords = kNear / 32 + kFilterWords + kTail;  // a warp's shared memory in the far kernel
+// A warp claims kSegment units of work, a record being one.  A near row adds
+// kNearWeight (setting and clearing its bitmap: records alone took a graph of
+// 2^14 rows 2x as long, 256 the mixed batch 3% longer), a far row kRowWeight
+// (32 short ones are handled together).
+constexpr uint32_t kSegment = 512;
+constexpr int kNearWeight = 128;
+constexpr int kRowWeight = 4;
+// Blocks an SM and 16-byte vectors per lane in flight when probing (near:
+// 6 and 2 1470 us, 4 and 4 1375, 5 and 3 1336; far: 5 and 2 spill, 1420 us,
+// 4 and 2 1195, 4 and 3 1167).
+constexpr int kNearBlocksPerSm = 5;
+constexpr int kNearInFlight = 3;
+constexpr int kFarBlocksPerSm = 4;
+constexpr int kFarInFlight = 3;
 constexpr int kUnroll = 2;        // the scan's rounds of 32 nonzeros in flight per warp (4 spill: 510 against 375 us)
 constexpr int kHub = 8192;        // labels whose incoming counts and slots live in shared memory
 constexpr int kScanBlocksPerSm = 3;
 constexpr uint32_t kChunkMin = 256;     // nonzeros of a chunk at least: two rounds of the fill
 constexpr uint32_t kChunksPerWarp = 4;  // chunks a warp takes in turn when the scan fills the GPU
-constexpr int kFillUnroll = 4;     // the fill's rounds in flight (chunks are a multiple of them)
-constexpr int kProbeInFlight = 5;  // 16-byte prefix vectors per lane in flight when probing
+constexpr int kFillUnroll = 2;     // the fill's rounds in flight (chunks are a multiple of them)
 constexpr int kStagedInFlight = 2; // the same for prefixes probed against staged short rows
 constexpr int kDenseHubs = 16384;  // rows j below this keep a bitmap of their columns for dense pairs
 constexpr int kDenseThreads = 256;
@@ -92,7 +119,8 @@ __device__ __forceinline__ bool dense_pair(uint32_t j, uint32_t p, int64_t ov, u
 }
 
 struct Layout {
-  size_t col32, in_cnt, in_off, bsum, in_rec, hubs, bits, starts, words, total;
+  size_t col32, rows16, nlow, in_cnt, in_off, bsum, in_rec, hubs, bits, starts, words, total;
+  size_t nvec16;        // 16-byte vectors of rows16, the last one pads
   uint32_t dense_hubs;  // rows with a column bitmap: min(kDenseHubs, numrows rounded up to 128)
   uint32_t chunk;       // nonzeros per chunk of the scan and the fill (a multiple of a warp's round)
   uint32_t nchunks;
@@ -101,12 +129,22 @@ struct Layout {
 
 size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// log2 of a warp's bitmap: min(kNearBits, labels rounded up to a power of two >= 32).
+int warp_bits(int64_t numrows) {
+  int wb = 5;
+  while (wb < kNearBits && (int64_t(1) << wb) < numrows) wb++;
+  return wb;
+}
+
 Layout layout(int64_t n, int64_t nnz) {
   Layout l;
   const size_t nz = static_cast<size_t>(nnz > 0 ? nnz : 1);
   const size_t nb = static_cast<size_t>((n + kPsumBlock - 1) / kPsumBlock) + 1;
   size_t o = 0;
   l.col32 = o;  o += up256(nz * 4);
+  l.nvec16 = nz / 8 + static_cast<size_t>(n) + 1;
+  l.rows16 = o; o += up256(l.nvec16 * 16);
+  l.nlow = o;   o += up256(static_cast<size_t>(n) * 4);
   l.in_cnt = o; o += up256(static_cast<size_t>(n) * 4 + 4);
   l.in_off = o; o += up256(static_cast<size_t>(n + 1) * 4);
   l.bsum = o;   o += up256(nb * 4);
@@ -115,7 +153,8 @@ Layout layout(int64_t n, int64_t nnz) {
   // kChunksPerWarp of them, longer ones beyond that
   const size_t warps = static_cast<size_t>(num_sms()) * kScanBlocksPerSm * kScanWarps;
   const size_t want = (nz + warps * kChunksPerWarp - 1) / (warps * kChunksPerWarp);
-  l.chunk = static_cast<uint32_t>(std::max<size_t>(kChunkMin, (want + 32 * kFillUnroll - 1) / (32 * kFillUnroll) * (32 * kFillUnroll)));
+  constexpr size_t round = 32 * kFillUnroll;
+  l.chunk = static_cast<uint32_t>(std::max<size_t>(kChunkMin, (want + round - 1) / round * round));
   l.nchunks = static_cast<uint32_t>((nz + l.chunk - 1) / l.chunk);
   l.blocks = static_cast<uint32_t>(std::min<size_t>((l.nchunks + kScanWarps - 1) / kScanWarps,
                                                     static_cast<size_t>(num_sms()) * kScanBlocksPerSm));
@@ -164,22 +203,39 @@ __device__ __forceinline__ int flat_owner(uint32_t inc, uint32_t bb) {
   return o < 32u ? static_cast<int>(o) : 31;
 }
 
+// rows16 holds the rows' columns as 16 bits each, every row from a 16-byte
+// vector of its own on, row i (which starts at nonzero b) from vector
+// b / 8 + i: a row of d columns needs at most d / 8 + 1 of them, and the next
+// row's start is that far on.  Columns that are not low read as `pad`, and so
+// do the places behind a row's end in its last vector.  No bitmap has the
+// pad's bit set (row j's columns lie below j, and low rows' below the pad's
+// label), and the columns of row i from j on are not in row j either: whole
+// vectors are probed, with no test of where the prefix or the row ends.
+__device__ __forceinline__ uint64_t vec16(uint32_t b, int64_t i) {
+  return static_cast<uint64_t>(b >> 3) + static_cast<uint64_t>(i);
+}
+
 // Row offsets: rows outside [0,nnz] or descending are counted (the later
 // kernels then return before they use any), the incoming counts are zeroed,
+// nlow[i] (the place of row i's first column that is not low) is set to none,
 // and starts[c] becomes the row that holds nonzero c * chunk -- so the scan
 // and the fill can split the nonzeros evenly, whatever the rows' lengths.
 // Chunks before the first row's start begin at row 0, those past the last
 // row's end at row n (no rows).
 __global__ void __launch_bounds__(kRowsThreads)
     wedge_rows_kernel(const int64_t *__restrict__ off, int64_t n, int64_t nnz, uint32_t *__restrict__ in_cnt,
+                      uint32_t *__restrict__ nlow, uint4 *__restrict__ rows16, uint64_t nvec16, uint32_t pad,
                       uint32_t *__restrict__ starts, uint32_t chunk, uint32_t nchunks,
                       unsigned long long *__restrict__ words, unsigned long long *__restrict__ bad,
                       const unsigned *__restrict__ run_if) {
   if (tri::skipped(run_if, 1u)) return;
   unsigned long long nbad = 0;
+  const uint32_t pads = pad | (pad << 16);
+  if (blockIdx.x == 0 && threadIdx.x == 0) rows16[nvec16 - 1] = make_uint4(pads, pads, pads, pads);
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kRowsThreads;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * kRowsThreads + threadIdx.x; i < n; i += stride) {
     in_cnt[i] = 0;
+    nlow[i] = 0xffffffffu;
     const int64_t b = off[i], e = off[i + 1];
     if (b < 0 || e < b || e > nnz) {
       nbad++;
@@ -187,6 +243,8 @@ __global__ void __launch_bounds__(kRowsThreads)
     }
     // nnz < 2^32 - 256, so offsets and chunk starts fit 32 bits
     const uint32_t b32 = static_cast<uint32_t>(b), e32 = static_cast<uint32_t>(e);
+    // the scan fills in the last vector's columns
+    if (e32 - b32 > 1) rows16[vec16(b32, i) + (e32 - b32 - 1) / 8] = make_uint4(pads, pads, pads, pads);
     uint32_t c = b32 / chunk + (b32 % chunk ? 1u : 0u);
     if (i == 0)
       for (uint32_t t = 0; t < c && t < nchunks; t++) starts[t] = 0;
@@ -239,14 +297,15 @@ struct RowWindow {
   }
 };
 
-// The row r of [lo,n) with off[r] <= k < off[r + 1], for ascending offsets
-// with off[lo] <= k < off[n] (whole warp; 32 places tested per step).
-__device__ __forceinline__ int64_t row_of(const int64_t *__restrict__ off, int64_t lo, int64_t n, int64_t k) {
+// The row r of [lo,n) with off(r) <= k < off(r + 1), for ascending offsets
+// with off(lo) <= k < off(n) (whole warp; 32 places tested per step).
+template <class Offset>
+__device__ __forceinline__ int64_t row_of(Offset off, int64_t lo, int64_t n, int64_t k) {
   int64_t hi = n;
   while (hi - lo > 1) {
     const int64_t step = (hi - lo + 31) / 32;
     const int64_t at = lo + (static_cast<int64_t>(lane_id()) + 1) * step;
-    const int64_t c = __popc(__ballot_sync(kFull, at < hi && off[at] <= k));
+    const int64_t c = __popc(__ballot_sync(kFull, at < hi && off(at) <= k));
     const int64_t up = lo + (c + 1) * step;
     lo += c * step;
     hi = up < hi ? up : hi;
@@ -284,7 +343,7 @@ __device__ __forceinline__ void for_windows(const int64_t *__restrict__ off, int
     e = ne;
     if (__reduce_max_sync(kFull, e) <= end && r0 + 32 < n) {  // an empty window
       if (static_cast<int64_t>(end) >= off[n]) return;
-      r0 = row_of(off, r0, n, end);
+      r0 = row_of([off](int64_t i) { return off[i]; }, r0, n, end);
       b = e = 0;
       if (r0 + lane < n) {
         b = static_cast<uint32_t>(off[r0 + lane]);
@@ -336,7 +395,8 @@ __device__ __forceinline__ uint32_t take_global(uint32_t *a, bool on) {
 __global__ void __launch_bounds__(kScanThreads, kScanBlocksPerSm)
     wedge_scan_kernel(const int64_t *__restrict__ off, const int64_t *__restrict__ col, int64_t n, int64_t nnz,
                       const uint32_t *__restrict__ starts, uint32_t chunk, uint32_t nchunks,
-                      uint32_t *__restrict__ col32, uint32_t *__restrict__ in_cnt, uint32_t *__restrict__ hubs,
+                      uint32_t *__restrict__ col32, uint16_t *__restrict__ rows16, uint32_t pad,
+                      uint32_t *__restrict__ nlow, uint32_t *__restrict__ in_cnt, uint32_t *__restrict__ hubs,
                       unsigned long long *__restrict__ words, unsigned long long *__restrict__ bad, int64_t ov,
                       uint32_t dhubs, const unsigned *__restrict__ run_if) {
   if (tri::skipped(run_if, 1u)) return;
@@ -378,8 +438,13 @@ __global__ void __launch_bounds__(kScanThreads, kScanBlocksPerSm)
           const uint32_t end = __shfl_sync(kFull, u == 0 ? carry : cu[u > 0 ? u - 1 : 0], 31);
           if (lane == 0) prv = end;
           const bool in = base + 32 * u + lane < w.tot;
-          const bool ok = cu[u] < static_cast<uint32_t>(r0) + r[u] && (p[u] == 0 || cu[u] > prv);
-          if (in) col32[k[u]] = ok ? cu[u] : kBadCol;
+          const uint32_t i = static_cast<uint32_t>(r0) + r[u];
+          const bool ok = cu[u] < i && (p[u] == 0 || cu[u] > prv);
+          if (in) {
+            col32[k[u]] = ok ? cu[u] : kBadCol;
+            rows16[vec16(k[u] - p[u], i) * 8 + p[u]] = static_cast<uint16_t>(cu[u] < pad ? cu[u] : pad);
+            if (cu[u] >= kLow && (p[u] == 0 || prv < kLow)) nlow[i] = p[u];
+          }
           nbad += in && !ok;
           const bool inner = in && ok && p[u] > 0;
           const bool dense = inner && dense_pair(cu[u], p[u], ov, dhubs);
@@ -543,13 +608,12 @@ __global__ void __launch_bounds__(kScanThreads, kScanBlocksPerSm)
   for (uint32_t ch = blockIdx.x * kScanWarps + (threadIdx.x >> 5); ch < nchunks; ch += warps) {
     const uint32_t k0 = ch * chunk;
     const uint32_t k1 = static_cast<uint32_t>(nnz) - k0 < chunk ? static_cast<uint32_t>(nnz) : k0 + chunk;
-    for_windows(off, n, starts[ch], k0, k1, stage[threadIdx.x >> 5], [&](const RowWindow &w, int64_t) {
+    for_windows(off, n, starts[ch], k0, k1, stage[threadIdx.x >> 5], [&](const RowWindow &w, int64_t r0) {
       for (uint32_t base = 0; base < w.tot; base += 32 * kFillUnroll) {
-        uint32_t k[kFillUnroll], p[kFillUnroll], c[kFillUnroll], slot[kFillUnroll];
+        uint32_t k[kFillUnroll], p[kFillUnroll], r[kFillUnroll], c[kFillUnroll], slot[kFillUnroll];
 #pragma unroll
         for (int u = 0; u < kFillUnroll; u++) {
-          uint32_t r;
-          w.at(base + 32 * u, k[u], p[u], r);
+          w.at(base + 32 * u, k[u], p[u], r[u]);
           c[u] = base + 32 * u + lane < w.tot ? col32[k[u]] : kBadCol;
           // the first nonzero of a row closes no wedge; dense pairs are counted apart
           if (p[u] == 0 || (c[u] != kBadCol && dense_pair(c[u], p[u], ov, dhubs))) c[u] = kBadCol;
@@ -562,71 +626,122 @@ __global__ void __launch_bounds__(kScanThreads, kScanBlocksPerSm)
         }
 #pragma unroll
         for (int u = 0; u < kFillUnroll; u++)
-          if (c[u] != kBadCol) in_rec[slot[u]] = make_uint2(k[u] - p[u], p[u]);
+          if (c[u] != kBadCol) {
+            // near j: p <= j < 2^15, and the vector index has 33 bits at most
+            const uint64_t v = vec16(k[u] - p[u], r0 + r[u]);
+            const uint32_t i = static_cast<uint32_t>(r0) + r[u];
+            const uint32_t top = static_cast<uint32_t>(v >> 32) << 16;
+            in_rec[slot[u]] = c[u] < kNear ? make_uint2(static_cast<uint32_t>(v), p[u] | top) : make_uint2(i, p[u]);
+          }
       }
     });
   }
 }
 
-// Is element w of an incoming prefix in row j?  Labels below `lim` are
-// tested in the bitmap; with OVF the others are searched in row j's sorted
-// tail [lim, j) -- kept in shared memory when it has at most kOvf entries.
-template <bool OVF>
-struct RowJ {
-  const uint32_t *bm;
-  uint32_t wmask, lim;
-  const uint32_t *tail;  // shared-memory copy, or the tail in col32
-  uint32_t ntail;
-  __device__ __forceinline__ uint32_t has(uint32_t w) const {
-    if (!OVF || w < lim) return tri::bit_of(bm, wmask, w);
-    return search_u32(tail, ntail, w) ? 1u : 0u;
-  }
-  // elements of x (element indices base..base+3) inside [s, s + len)
-  __device__ __forceinline__ uint32_t test4(uint4 x, uint32_t base, uint32_t s, uint32_t len) const {
-    const uint32_t o = base - s;  // wraps for elements before s
-    uint32_t c = 0;
-    if (o < len) c += has(x.x);
-    if (o + 1u < len) c += has(x.y);
-    if (o + 2u < len) c += has(x.z);
-    if (o + 3u < len) c += has(x.w);
-    return c;
-  }
-};
+// add + (v >> shift) in one instruction
+template <int SHIFT>
+__device__ __forceinline__ uint32_t shr_add(uint32_t v, uint32_t add) {
+  uint32_t r;
+  asm("mad.hi.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(v), "n"(1u << (32 - SHIFT)), "r"(add));
+  return r;
+}
 
-// Probes of up to 32 prefixes (lane l holds record l; {0,0} for none; real
-// records have p >= 1) against row j: every element of each prefix
-// row_i[s, s+p) is tested.  The prefixes' 16-byte vectors are flattened over
-// the warp so every lane has a vector whatever the prefix lengths,
-// kProbeInFlight vectors per lane in flight.
-template <bool OVF>
-__device__ __forceinline__ void probe_records(const RowJ<OVF> rj, const uint4 *__restrict__ col4, uint32_t nvec_all,
-                                              uint2 rec, unsigned long long &cnt, unsigned long long &wk) {
-  const unsigned lane = lane_id();
-  const uint32_t s = rec.x, p = rec.y;
-  const uint32_t v0 = s >> 2;
-  const uint32_t nv = p ? ((s + p + 3u) >> 2) - v0 : 0u;
-  const uint32_t inc = incl_scan_u32(nv);
-  const uint32_t tot = __shfl_sync(kFull, inc, 31);
-  const uint32_t q = v0 - (inc - nv);  // vector index = q + flattened position
-  wk += p;
-  for (uint32_t base = 0; base < tot; base += 32 * kProbeInFlight) {
-    uint4 xv[kProbeInFlight];
-    uint32_t vi[kProbeInFlight], ps[kProbeInFlight], pl[kProbeInFlight];
-    bool act[kProbeInFlight];
+__device__ __forceinline__ uint32_t lds(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+
+// Bitmap word and bit of a label: the words' bits run from the top, so that
+// a left shift by the label leaves its bit in the sign.
+__device__ __forceinline__ uint32_t low_bit(uint32_t c) { return 0x80000000u >> (c & 31u); }
+
+// cnt + the number of the eight 16-bit labels of x that are set in the
+// bitmap at shared-memory address bm.
+__device__ __forceinline__ uint32_t test8(uint32_t bm, uint4 x, uint32_t cnt) {
+  const uint32_t v[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-    for (int h = 0; h < kProbeInFlight; h++) {
-      const uint32_t bb = base + 32u * h;
-      const int o = flat_owner(inc, bb);
-      vi[h] = __shfl_sync(kFull, q, o) + bb + lane;
-      ps[h] = __shfl_sync(kFull, s, o);
-      pl[h] = __shfl_sync(kFull, p, o);
-      act[h] = bb + lane < tot && vi[h] < nvec_all;
-      xv[h] = act[h] ? col4[vi[h]] : make_uint4(0u, 0u, 0u, 0u);
+  for (int t = 0; t < 4; t++) {
+    const uint32_t w0 = lds(shr_add<3>(v[t] & 0xffe0u, bm));
+    const uint32_t w1 = lds(shr_add<19>(v[t] & 0xffe00000u, bm));
+    cnt = shr_add<31>(__funnelshift_l(0u, w0, v[t]), cnt);
+    cnt = shr_add<31>(__funnelshift_l(0u, w1, v[t] >> 16), cnt);
+  }
+  return cnt;
+}
+
+// Hits in the bitmap at bm among the vectors of nrec prefixes.  fetch(r)
+// gives lane l its prefix r + l: the first vector and their number nv (nv >= 1;
+// 0 in the lanes behind the last prefix).  The vectors of 32 prefixes are
+// flattened over the warp, so every lane has one whatever the prefix lengths,
+// K vectors per lane in flight.  Lanes without a vector read the last one,
+// which is all pads.  WIDE: 2^32 vectors and more.  (Vectors asked for ahead
+// across the ends of the batches, one at a time or in pairs: 2806 -> 3180 and
+// 2660 us against 2610, the registers costing more than the waits.)
+template <bool WIDE, int K, class Fetch>
+__device__ __forceinline__ unsigned long long probe_stream(uint32_t bm, const uint4 *__restrict__ rows16,
+                                                           uint64_t nvec16, uint32_t nrec, Fetch fetch) {
+  using Index = typename std::conditional<WIDE, uint64_t, uint32_t>::type;
+  const unsigned lane = lane_id();
+  const Index pads = static_cast<Index>(nvec16 - 1);
+  uint32_t r = 0, base = 0, tot = 0, inc = 0;
+  Index q = 0;
+  const auto issue = [&](uint4 *x) -> bool {
+    if (base >= tot) {
+      if (r >= nrec) return false;
+      uint64_t v0 = 0;
+      const uint32_t nv = fetch(r, v0);
+      r += 32;
+      inc = incl_scan_u32(nv);
+      tot = __shfl_sync(kFull, inc, 31);
+      q = static_cast<Index>(v0) - (inc - nv);  // vector index = q + flattened position
+      base = 0;
     }
 #pragma unroll
-    for (int h = 0; h < kProbeInFlight; h++)
-      if (act[h]) cnt += rj.test4(xv[h], vi[h] << 2, ps[h], pl[h]);
+    for (int h = 0; h < K; h++) {
+      const uint32_t bb = base + 32u * h;
+      Index v = __shfl_sync(kFull, q, flat_owner(inc, bb)) + (bb + lane);
+      v = bb + lane < tot && v < pads ? v : pads;
+      x[h] = rows16[v];
+    }
+    base += 32 * K;
+    return true;
+  };
+  const auto test = [&](const uint4 *x) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int h = 0; h < K; h++) c = test8(bm, x[h], c);
+    return c;
+  };
+  uint4 x[K];
+  unsigned long long total = 0;
+  while (issue(x)) total += test(x);
+  return total;
+}
+
+// The filter of a far row's columns that are not low: their low 12 bits.
+__device__ __forceinline__ uint32_t filter_word(uint32_t c) { return (c >> 5) & (kFilterWords - 1); }
+
+// The elements of up to 32 runs of columns (lane l holds run [s, s + c), c >= 1
+// but in the lanes behind the last) that are in the ascending list
+// tail[0,ntail), whose columns are set in the filter: whole warp, the runs
+// flattened over the lanes.
+__device__ __forceinline__ uint32_t probe_tail(const uint32_t *filter, const uint32_t *__restrict__ tail,
+                                               uint32_t ntail, const uint32_t *__restrict__ col32, uint32_t s,
+                                               uint32_t c) {
+  const unsigned lane = lane_id();
+  const uint32_t inc = incl_scan_u32(c);
+  const uint32_t tot = __shfl_sync(kFull, inc, 31);
+  const uint32_t q = s - (inc - c);
+  uint32_t cnt = 0;
+  for (uint32_t base = 0; base < tot; base += 32) {
+    const uint32_t k = __shfl_sync(kFull, q, flat_owner(inc, base)) + base + lane;
+    if (base + lane < tot) {
+      const uint32_t w = col32[k];
+      if ((filter[filter_word(w)] & low_bit(w)) && search_u32(tail, ntail, w)) cnt++;
+    }
   }
+  return cnt;
 }
 
 // Probes of up to 32 prefixes of different rows j (lane l holds record l
@@ -684,79 +799,131 @@ __device__ __forceinline__ void flush(unsigned long long cnt, unsigned long long
   }
 }
 
-// One warp per row j, each warp with its own bitmap of 2^wbits labels and a
-// kOvf-entry tail list in shared memory.  Rows below wlim = min(n, 2^wbits)
-// (all columns inside the bitmap) are claimed one at a time in label order,
-// which on a degree-ordered matrix starts with the rows that close the most
-// wedges; the rest 32 at a time, one lane checking each for incoming
-// prefixes so that empty ones cost no serial loads.
-__global__ void __launch_bounds__(kWarpThreads, 3)
-    wedge_count_kernel(const int64_t *__restrict__ off, const uint32_t *__restrict__ col32,
-                       const uint32_t *__restrict__ in_off, const uint2 *__restrict__ in_rec, int64_t n, int64_t wlim,
-                       int wbits, uint32_t nvec_all, uint32_t stage_max, const unsigned long long *__restrict__ words,
-                       unsigned long long *__restrict__ count, unsigned long long *__restrict__ work,
-                       unsigned long long *__restrict__ cursor, const unsigned *__restrict__ run_if) {
+// The near rows j, below rows = min(n, kNear): a warp claims kSegment units of
+// the records and the rows' weights, row j's units being place(j) up to
+// place(j + 1), its records first; a row may be cut between claims.
+template <bool WIDE>
+__global__ void __launch_bounds__(kWarpThreads, kNearBlocksPerSm)
+    wedge_near_kernel(const int64_t *__restrict__ off, const uint32_t *__restrict__ col32,
+                      const uint4 *__restrict__ rows16, uint64_t nvec16, const uint32_t *__restrict__ in_off,
+                      const uint2 *__restrict__ in_rec, uint32_t rows, int nearbits,
+                      const unsigned long long *__restrict__ words, unsigned long long *__restrict__ count,
+                      unsigned long long *__restrict__ work, unsigned long long *__restrict__ cursor,
+                      const unsigned *__restrict__ run_if) {
   if (tri::skipped(run_if, 1u)) return;
   extern __shared__ uint32_t wsm[];
   if (words[kWBad]) return;
   const unsigned lane = lane_id();
-  const uint32_t nw = 1u << (wbits - 5);
-  uint32_t *bm = wsm + static_cast<size_t>(threadIdx.x >> 5) * (nw + kOvf);
-  uint32_t *ovf = bm + nw;
-  const uint32_t lim = 1u << wbits;
-  const uint4 *__restrict__ col4 = reinterpret_cast<const uint4 *>(col32);  // col32 is 256-byte aligned
+  const uint32_t nw = 1u << (nearbits - 5);
+  uint32_t *bm = wsm + static_cast<size_t>(threadIdx.x >> 5) * nw;
+  const uint32_t bma = static_cast<uint32_t>(__cvta_generic_to_shared(bm));
   for (uint32_t w = lane; w < nw; w += 32) bm[w] = 0;
   __syncwarp();
   unsigned long long cnt = 0, wk = 0;
-  const unsigned long long nbig = static_cast<unsigned long long>(wlim);
-  // Two queues: rows below wlim one at a time (cursor[0], issue-bound work)
-  // and claims of 32 rows above it (cursor[1], latency-bound); each warp
-  // alternates between them so that the two kinds overlap on every SM.
-  bool big_done = false, small_done = false;
-  for (unsigned it = 0;; it++) {
-    if (big_done && small_done) break;
-    const bool take_big = !big_done && (small_done || (it & 1u) == 0);
+  const auto place = [in_off](int64_t j) {
+    return static_cast<int64_t>(in_off[j]) + j * static_cast<int64_t>(kNearWeight);
+  };
+  const int64_t all = place(rows);
+  for (;;) {
     unsigned long long t = 0;
-    if (lane == 0) t = atomicAdd(cursor + (take_big ? 0 : 1), 1ull);
-    t = __shfl_sync(kFull, t, 0);
-    int64_t j0, j1;
-    if (take_big) {
-      if (t >= nbig) {
-        big_done = true;
-        continue;
+    if (lane == 0) t = atomicAdd(cursor, 1ull);
+    const int64_t s0 = static_cast<int64_t>(__shfl_sync(kFull, t, 0)) * kSegment;
+    if (s0 >= all) break;
+    const int64_t s1 = s0 + kSegment;
+    for (int64_t j = row_of(place, 0, rows, s0), to = s0; j < rows && to < s1; j++) {
+      const int64_t w = j * static_cast<int64_t>(kNearWeight);
+      const int64_t from = in_off[j], upto = in_off[j + 1];
+      to = upto + w + kNearWeight;
+      const int64_t lo = s0 - w > from ? s0 - w : from, hi = s1 - w < upto ? s1 - w : upto;
+      const uint32_t b = static_cast<uint32_t>(off[j]), d = static_cast<uint32_t>(off[j + 1]) - b;
+      if (hi <= lo || d == 0) continue;
+      const uint32_t r0 = static_cast<uint32_t>(lo), nrec = static_cast<uint32_t>(hi - lo);
+      for (uint32_t k = lane; k < d; k += 32) {
+        const uint32_t c = col32[b + k];
+        atomicOr(&bm[(c >> 5) & (nw - 1u)], low_bit(c));
       }
-      j0 = static_cast<int64_t>(t);
-      j1 = j0 + 1;
-    } else {
-      j0 = wlim + static_cast<int64_t>(t) * 32;
-      if (j0 >= n) {
-        small_done = true;
-        continue;
+      __syncwarp();
+      uint2 next = lane < nrec ? in_rec[r0 + lane] : make_uint2(0u, 0u);
+      cnt += probe_stream<WIDE, kNearInFlight>(bma, rows16, nvec16, nrec, [&](uint32_t r, uint64_t &v0) {
+        const uint2 rec = next;
+        next = r + 32 + lane < nrec ? in_rec[r0 + r + 32 + lane] : make_uint2(0u, 0u);
+        const uint32_t p = rec.y & 0xffffu;
+        v0 = rec.x | (WIDE ? static_cast<uint64_t>(rec.y >> 16) << 32 : uint64_t(0));
+        wk += p;
+        return (p + 7u) >> 3;
+      });
+      __syncwarp();
+      for (uint32_t k = lane; k < d; k += 32) bm[(col32[b + k] >> 5) & (nw - 1u)] = 0;
+      __syncwarp();
+    }
+  }
+  flush(cnt, wk, count, work);
+}
+
+// The far rows j, from kNear on, claimed in the same way but looked at 32 at a
+// time, one lane each, so that rows without records cost no serial loads.  A
+// warp has a bitmap of the low labels, the filter of row j's other columns
+// and room for kTail of them.
+template <bool WIDE>
+__global__ void __launch_bounds__(kWarpThreads, kFarBlocksPerSm)
+    wedge_far_kernel(const int64_t *__restrict__ off, const uint32_t *__restrict__ col32,
+                     const uint4 *__restrict__ rows16, uint64_t nvec16, const uint32_t *__restrict__ nlow,
+                     const uint32_t *__restrict__ in_off, const uint2 *__restrict__ in_rec, int64_t n,
+                     uint32_t nvec_all, uint32_t stage_max, const unsigned long long *__restrict__ words,
+                     unsigned long long *__restrict__ count, unsigned long long *__restrict__ work,
+                     unsigned long long *__restrict__ cursor, const unsigned *__restrict__ run_if) {
+  if (tri::skipped(run_if, 1u)) return;
+  extern __shared__ uint32_t wsm[];
+  if (words[kWBad]) return;
+  const unsigned lane = lane_id();
+  constexpr int64_t near = kNear;
+  constexpr uint32_t nw = kNear / 32;
+  uint32_t *bm = wsm + static_cast<size_t>(threadIdx.x >> 5) * kFarWords;
+  uint32_t *filter = bm + nw;
+  uint32_t *list = filter + kFilterWords;
+  const uint32_t bma = static_cast<uint32_t>(__cvta_generic_to_shared(bm));
+  const uint4 *__restrict__ col4 = reinterpret_cast<const uint4 *>(col32);  // col32 is 256-byte aligned
+  for (uint32_t w = lane; w < nw + kFilterWords; w += 32) bm[w] = 0;
+  __syncwarp();
+  unsigned long long cnt = 0, wk = 0;
+  const auto place = [in_off](int64_t j) {
+    return static_cast<int64_t>(in_off[j]) + (j - near) * static_cast<int64_t>(kRowWeight);
+  };
+  const int64_t first = in_off[near], all = place(n);
+  for (;;) {
+    unsigned long long t = 0;
+    if (lane == 0) t = atomicAdd(cursor, 1ull);
+    const int64_t s0 = first + static_cast<int64_t>(__shfl_sync(kFull, t, 0)) * kSegment;
+    if (s0 >= all) break;
+    const int64_t s1 = s0 + kSegment;
+    for (int64_t j0 = row_of(place, near, n, s0), to = s0; j0 < n && to < s1;) {
+      // rows of this window with incoming prefixes in the segment and a non-empty row j
+      const int64_t jl = j0 + lane;
+      bool live = false;
+      uint32_t lb = 0, ld = 0, lr0 = 0, lnr = 0;
+      if (jl < n) {
+        const int64_t w = (jl - near) * static_cast<int64_t>(kRowWeight);
+        const int64_t from = in_off[jl], upto = in_off[jl + 1];
+        const int64_t lo = s0 - w > from ? s0 - w : from, hi = s1 - w < upto ? s1 - w : upto;
+        lr0 = static_cast<uint32_t>(lo);
+        lnr = hi > lo ? static_cast<uint32_t>(hi - lo) : 0u;
+        const int64_t bb = off[jl], dd = off[jl + 1] - bb;
+        live = lnr > 0 && dd > 0;
+        lb = static_cast<uint32_t>(bb);
+        ld = static_cast<uint32_t>(dd);
+        to = upto + w + kRowWeight;
       }
-      j1 = j0 + 32 < n ? j0 + 32 : n;
-    }
-    // rows of this claim with incoming prefixes and a non-empty row j
-    const int64_t jl = j0 + lane;
-    bool live = false;
-    uint32_t lb = 0, ld = 0, lr0 = 0, lnr = 0;
-    if (jl < j1) {
-      lr0 = in_off[jl];
-      lnr = in_off[jl + 1] - lr0;
-      const int64_t bb = off[jl], dd = off[jl + 1] - bb;
-      live = lnr > 0 && dd > 0;
-      lb = static_cast<uint32_t>(bb);
-      ld = static_cast<uint32_t>(dd);
-    }
-    if (!take_big) {
-      // Rows above wlim: the short ones (at most stage_max columns, where a
+      to = __shfl_sync(kFull, to, 31);  // where the next window begins (j0 + 32 < n)
+      j0 += 32;
+      // The short rows (at most stage_max columns, where a
       // binary search beats setting and clearing a bitmap) are staged in the
       // warp's buffer -- as many at a time as fit -- and all their prefixes
-      // probed flattened, so they cost a few memory round trips per claim
-      // instead of a few per row.  The bitmap area is the buffer, zeroed
+      // probed flattened, so they cost a few memory round trips per window
+      // instead of a few per row.  The bitmap is the buffer, zeroed
       // again after each batch.
-      uint4 *slot = reinterpret_cast<uint4 *>(ovf + kOvf) - 32;
+      uint4 *slot = reinterpret_cast<uint4 *>(list);
       uint32_t *stg = bm;
-      const uint32_t cap = nw + kOvf - 128;
+      constexpr uint32_t cap = nw;
       const bool fits = live && ld <= stage_max;
       const unsigned lm = __ballot_sync(kFull, fits);
       if (fits) slot[__popc(lm & ((1u << lane) - 1u))] = make_uint4(lb, ld, lr0, lnr);
@@ -790,7 +957,11 @@ __global__ void __launch_bounds__(kWarpThreads, 3)
           const int o = flat_owner(incr, base);
           const uint32_t o0 = __shfl_sync(kFull, cr0, o), ox = __shfl_sync(kFull, incr - cn, o);
           const uint32_t ro = __shfl_sync(kFull, incd - cd, o) - base_s, rl = __shfl_sync(kFull, cd, o);
-          const uint2 rec = base + lane < totr ? in_rec[o0 + (base + lane - ox)] : make_uint2(0u, 0u);
+          uint2 rec = make_uint2(0u, 0u);
+          if (base + lane < totr) {
+            rec = in_rec[o0 + (base + lane - ox)];
+            rec.x = static_cast<uint32_t>(off[rec.x]);
+          }
           probe_records_staged(stg, ro, rl, col4, nvec_all, rec, cnt, wk);
         }
         __syncwarp();
@@ -798,55 +969,53 @@ __global__ void __launch_bounds__(kWarpThreads, 3)
         __syncwarp();
         t0 = t1;
       }
-      // longer rows: one at a time below, on the (zero) bitmap
       live = live && !fits;
-      if (!__any_sync(kFull, live)) continue;
-    }
-    unsigned todo = __ballot_sync(kFull, live);
-    while (todo) {
-      const int64_t j = j0 + __ffs(todo) - 1;
-      todo &= todo - 1;
-      const uint32_t r0 = in_off[j], nrec = in_off[j + 1] - r0;
-      const int64_t b = off[j], d = off[j + 1] - b;
-      if (j < wlim) {
-        for (int64_t k = lane; k < d; k += 32) {
-          const uint32_t c = col32[b + k];
-          atomicOr(&bm[(c >> 5) & (nw - 1u)], 1u << (c & 31));
-        }
-        __syncwarp();
-        const RowJ<false> rj{bm, nw - 1u, lim, nullptr, 0u};
-        for (uint32_t r = 0; r < nrec; r += 32) {
-          const uint2 rec = r + lane < nrec ? in_rec[r0 + r + lane] : make_uint2(0u, 0u);
-          probe_records(rj, col4, nvec_all, rec, cnt, wk);
-        }
-      } else {
-        // columns below lim go to the bitmap, the ascending tail [lim, j) to the list
+      // longer rows: one at a time, on the (zero) bitmap
+      unsigned todo = __ballot_sync(kFull, live);
+      while (todo) {
+        const int at = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const uint32_t r0 = __shfl_sync(kFull, lr0, at), nrec = __shfl_sync(kFull, lnr, at);
+        const uint32_t b = __shfl_sync(kFull, lb, at), d = __shfl_sync(kFull, ld, at);
+        uint2 next = lane < nrec ? in_rec[r0 + lane] : make_uint2(0u, 0u);
+        // row j's low columns go to the bitmap, the others (its ascending tail) to the filter
         uint32_t below = 0;
-        for (int64_t k = lane; k < d; k += 32) {
+        for (uint32_t k = lane; k < d; k += 32) {
           const uint32_t c = col32[b + k];
-          if (c < lim) {
-            atomicOr(&bm[c >> 5], 1u << (c & 31));
-            below++;
-          }
+          atomicOr(c < kLow ? &bm[c >> 5] : &filter[filter_word(c)], low_bit(c));
+          below += c < kLow;
         }
         below = __reduce_add_sync(kFull, below);
-        const uint32_t ntail = static_cast<uint32_t>(d) - below;
-        const bool cached = ntail <= static_cast<uint32_t>(kOvf);
+        const uint32_t ntail = d - below;
+        const bool cached = ntail <= static_cast<uint32_t>(kTail);
         if (cached)
-          for (uint32_t k = lane; k < ntail; k += 32) ovf[k] = col32[b + below + k];
+          for (uint32_t k = lane; k < ntail; k += 32) list[k] = col32[b + below + k];
         __syncwarp();
-        const RowJ<true> rj{bm, nw - 1u, lim, cached ? ovf : col32 + b + below, ntail};
-        for (uint32_t r = 0; r < nrec; r += 32) {
-          const uint2 rec = r + lane < nrec ? in_rec[r0 + r + lane] : make_uint2(0u, 0u);
-          probe_records(rj, col4, nvec_all, rec, cnt, wk);
+        cnt += probe_stream<WIDE, kFarInFlight>(bma, rows16, nvec16, nrec, [&](uint32_t r, uint64_t &v0) {
+          const uint2 rec = next;
+          next = r + 32 + lane < nrec ? in_rec[r0 + r + 32 + lane] : make_uint2(0u, 0u);
+          const uint32_t p = rec.y;
+          uint32_t start = 0, low = 0;
+          if (p) {
+            start = static_cast<uint32_t>(off[rec.x]);
+            low = nlow[rec.x] < p ? nlow[rec.x] : p;
+          }
+          v0 = vec16(start, rec.x);
+          wk += p;
+          // a prefix with no high column gives j itself, at place p, which row j does not have
+          const uint32_t high = p ? (p > low ? p - low : 1u) : 0u;
+          if (ntail)
+            cnt += cached ? probe_tail(filter, list, ntail, col32, start + low, high)
+                          : probe_tail(filter, col32 + b + below, ntail, col32, start + low, high);
+          return p ? (low + (low ? 7u : 8u)) >> 3 : 0u;  // with no low column still a vector (of pads)
+        });
+        __syncwarp();
+        for (uint32_t k = lane; k < d; k += 32) {
+          const uint32_t c = col32[b + k];
+          *(c < kLow ? &bm[c >> 5] : &filter[filter_word(c)]) = 0;
         }
+        __syncwarp();
       }
-      __syncwarp();
-      for (int64_t k = lane; k < d; k += 32) {
-        const uint32_t c = col32[b + k];
-        if (c < lim) bm[(c >> 5) & (nw - 1u)] = 0;
-      }
-      __syncwarp();
     }
   }
   flush(cnt, wk, count, work);
@@ -979,17 +1148,6 @@ __global__ void __launch_bounds__(kDenseThreads)
   flush(cnt, wk, count, work);
 }
 
-bool g_count_attr[64];
-
-// log2 of the per-warp bitmap: min(16, labels rounded up to a power of two >= 32).
-int warp_bits(int64_t numrows) {
-  int wb = 5;
-  while (wb < kWarpBitsMax && (int64_t(1) << wb) < numrows) wb++;
-  return wb;
-}
-
-size_t count_smem(int wb) { return ((size_t(1) << (wb - 5)) + kOvf) * sizeof(uint32_t) * kWarpWarps; }
-
 }  // namespace
 
 bool tri_wedge_supported(int64_t numrows, int64_t nnz) {
@@ -1013,16 +1171,20 @@ int tri_wedge_prepare(const int64_t *offset, const int64_t *nonzero, int64_t num
   uint32_t *bits = reinterpret_cast<uint32_t *>(p + l.bits);
   unsigned long long *words = reinterpret_cast<unsigned long long *>(p + l.words);
   uint32_t *starts = reinterpret_cast<uint32_t *>(p + l.starts);
+  uint32_t *nlow = reinterpret_cast<uint32_t *>(p + l.nlow);
+  const uint32_t pad = (1u << warp_bits(numrows)) - 1u;
   // dense pairs (tri.dense 0: none) and their margin over the bitmap's words
   const int64_t ov = knob_or("tri.dense", 1) == 0 ? -1 : knob_or("tri.dense_ov", 32);
   BALE_CUDA_OK(cudaMemsetAsync(words, 0, kWords * sizeof(unsigned long long), stream));
   const int64_t rblocks = std::min<int64_t>((numrows + kRowsThreads - 1) / kRowsThreads,
                                             static_cast<int64_t>(num_sms()) * kRowsBlocksPerSm);
   wedge_rows_kernel<<<static_cast<unsigned>(rblocks), kRowsThreads, 0, stream>>>(
-      offset, numrows, nnz, in_cnt, starts, l.chunk, l.nchunks, words, bad, run_if);
+      offset, numrows, nnz, in_cnt, nlow, reinterpret_cast<uint4 *>(p + l.rows16), l.nvec16, pad, starts, l.chunk,
+      l.nchunks, words, bad, run_if);
   BALE_CUDA_OK(cudaGetLastError());
-  wedge_scan_kernel<<<l.blocks, kScanThreads, 0, stream>>>(offset, nonzero, numrows, nnz, starts, l.chunk, l.nchunks,
-                                                           col32, in_cnt, hubs, words, bad, ov, l.dense_hubs, run_if);
+  wedge_scan_kernel<<<l.blocks, kScanThreads, 0, stream>>>(
+      offset, nonzero, numrows, nnz, starts, l.chunk, l.nchunks, col32, reinterpret_cast<uint16_t *>(p + l.rows16), pad,
+      nlow, in_cnt, hubs, words, bad, ov, l.dense_hubs, run_if);
   BALE_CUDA_OK(cudaGetLastError());
   if (ov >= 0 && l.dense_hubs > 0) {
     wedge_hubbits_kernel<<<static_cast<unsigned>((l.dense_hubs + 7) / 8), 256, 0, stream>>>(offset, col32, numrows,
@@ -1058,29 +1220,33 @@ int tri_wedge_run(const int64_t *offset, const void *ws, int64_t numrows, int64_
   const uint32_t *bits = reinterpret_cast<const uint32_t *>(p + l.bits);
   const unsigned long long *words = reinterpret_cast<const unsigned long long *>(p + l.words);
   const int sms = num_sms();
-  const int wb = warp_bits(numrows);
-  const int64_t wlim = numrows < (int64_t(1) << wb) ? numrows : (int64_t(1) << wb);
-  const uint32_t nvec_all = static_cast<uint32_t>((nnz + 3) / 4);
-  const uint32_t stage_max = static_cast<uint32_t>(knob_or("tri.wedge_stage_max", 64));
-  const size_t smem = count_smem(wb);
-  const int dev = current_device();
+  const int64_t near = std::min<int64_t>(numrows, kNear);
+  const bool wide = l.nvec16 >= (uint64_t(1) << 32);
+  const uint4 *rows16 = reinterpret_cast<const uint4 *>(p + l.rows16);
+  const auto warps_for = [sms](int64_t units, int per_sm) {
+    const int64_t claims = (units + kSegment - 1) / kSegment;
+    return static_cast<unsigned>(std::max<int64_t>(
+        1, std::min<int64_t>((claims + kWarpWarps - 1) / kWarpWarps, static_cast<int64_t>(sms) * per_sm)));
+  };
   BALE_CUDA_OK(cudaMemsetAsync(cursor, 0, 2 * sizeof(unsigned long long), stream));
-  if (dev >= 0 && dev < 64 && !g_count_attr[dev]) {
-    BALE_CUDA_OK(cudaFuncSetAttribute(wedge_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(count_smem(kWarpBitsMax))));
-    g_count_attr[dev] = true;
-  }
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wedge_count_kernel, kWarpThreads, smem) != cudaSuccess ||
-      occ < 1)
-    occ = 1;
-  int64_t blocks = static_cast<int64_t>(sms) * occ;
-  const int64_t claims = wlim + (numrows - wlim + 31) / 32;  // both queues
-  const int64_t need = (claims + kWarpWarps - 1) / kWarpWarps;
-  if (blocks > need) blocks = need > 0 ? need : 1;
-  wedge_count_kernel<<<static_cast<unsigned>(blocks), kWarpThreads, smem, stream>>>(
-      offset, col32, in_off, in_rec, numrows, wlim, wb, nvec_all, stage_max, words, count, work, cursor, run_if);
+  const int wb = warp_bits(numrows);
+  const auto near_kernel = wide ? wedge_near_kernel<true> : wedge_near_kernel<false>;
+  near_kernel<<<warps_for(nnz + near * kNearWeight, kNearBlocksPerSm), kWarpThreads,
+                (size_t(1) << (wb - 3)) * kWarpWarps, stream>>>(
+      offset, col32, rows16, l.nvec16, in_off, in_rec, static_cast<uint32_t>(near), wb, words, count, work, cursor,
+      run_if);
   BALE_CUDA_OK(cudaGetLastError());
+  if (near < numrows) {
+    const uint32_t nvec_all = static_cast<uint32_t>((nnz + 3) / 4);
+    const uint32_t stage_max =
+        static_cast<uint32_t>(std::min<int64_t>(knob_or("tri.wedge_stage_max", 64), kNear / 32));
+    const auto far_kernel = wide ? wedge_far_kernel<true> : wedge_far_kernel<false>;
+    far_kernel<<<warps_for(nnz + (numrows - near) * kRowWeight, kFarBlocksPerSm), kWarpThreads,
+                 kFarWords * sizeof(uint32_t) * kWarpWarps, stream>>>(
+        offset, col32, rows16, l.nvec16, reinterpret_cast<const uint32_t *>(p + l.nlow), in_off, in_rec, numrows,
+        nvec_all, stage_max, words, count, work, cursor + 1, run_if);
+    BALE_CUDA_OK(cudaGetLastError());
+  }
   // the dense pairs the prepare step left out of the records (none when its
   // margin was negative: the kernel returns at once)
   const int64_t dgroups = (numrows + kDenseThreads / 32 - 1) / (kDenseThreads / 32);

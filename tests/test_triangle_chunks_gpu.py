@@ -95,3 +95,26 @@ def test_malformed_matrices_count_nothing(cuda, bale, wedge, what):
     count, bad = torch.zeros(1, dtype=torch.int64, device=cuda), torch.zeros(1, dtype=torch.int64, device=cuda)
     bale.triangle_dev(torch.from_numpy(off).to(cuda), torch.from_numpy(col).to(cuda), count, bad=bad)
     assert int(bad.item()) > 0 and int(count.item()) == 0
+
+
+@pytest.mark.parametrize("n", [31, 32, 33, 4_096, 32_766, 32_767, 32_768, 32_769, 33_100, 65_600, 70_000])
+def test_rows_around_the_low_labels(cuda, bale, oracle, wedge, n):
+    """Rows and columns at both sides of 2^15 (near and far rows, low columns
+    and the list's, rows read in 16 bits), hubs with many prefixes, short far
+    rows beside long ones, and more other columns than the list holds."""
+    rng = np.random.default_rng(n)
+    edge = np.unique(np.clip(np.concatenate([np.arange(0, 40), np.arange(32_740, 32_800), np.arange(65_520, 65_560),
+                                             rng.integers(0, n, 300)]), 0, n - 1))
+    rows, off = [], np.zeros(n + 1, np.int64)
+    for i in range(n):
+        if i in (n - 1, n - 2, n - 3):  # long rows, all of whose columns are neighbours
+            r = edge[edge < i]
+            r = np.union1d(r, np.arange(max(0, i - 300), i))
+        elif i % 3 == 0 or i > n - 400:
+            below = edge[edge < i]
+            r = np.sort(rng.choice(below, min(below.size, int(rng.integers(0, 90))), replace=False))
+        else:
+            r = np.zeros(0, np.int64)
+        rows.append(r.astype(np.int64))
+        off[i + 1] = off[i] + r.size
+    _check(bale, oracle, off, np.concatenate(rows))

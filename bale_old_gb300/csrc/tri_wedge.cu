@@ -42,11 +42,11 @@
 //      warp (24 warps an SM) and a claim per row; 2806 with 16-bit rows; 2500
 //      as it is, near (40 warps an SM, its shared-memory data pipe 91% busy)
 //      1330 us and far (32 warps, waiting for dependent loads) 1170.
-//   5. dense pairs: a pair (i,j) whose prefix is longer than the ceil(j/32)
-//      words of a bitmap of [0,j) (plus a margin), for j below 2^14, gets no
+//   5. dense pairs: a pair (i,j) whose prefix is long against the ceil(j/32)
+//      words of a bitmap of [0,j) (dense_pair below), for j below 2^14, gets no
 //      record in steps 1-3; step 1 also builds the column bitmaps of the rows
-//      below 2^14, and one warp per row i ANDs row i's bits with row j's and
-//      counts them (54% of the scale-22 probes become 1.28 G word ANDs).
+//      below 2^14 and lists the rows i that have such pairs; warps claim these
+//      one by one, AND row i's bits with row j's and count them.
 // Steps 1-3 and the bitmaps depend only on the matrix (a resident graph does
 // them once).  A malformed row raises *bad in step 1 and the later steps then
 // return at once; every index stays inside its array either way.  The work
@@ -102,24 +102,29 @@ constexpr int kFillUnroll = 2;     // the fill's rounds in flight (chunks are a 
 constexpr int kStagedInFlight = 2; // the same for prefixes probed against staged short rows
 constexpr int kDenseHubs = 16384;  // rows j below this keep a bitmap of their columns for dense pairs
 constexpr int kDenseThreads = 256;
+constexpr int kDenseWarps = kDenseThreads / 32;
+constexpr int kDenseBlocksPerSm = 4;
 
 // Workspace words: [0] nonzero when the scan met a dense pair, [1] malformed
 // entries seen by the scan, [2] the dense-pair margin (negative: no dense
 // pairs), [3] the bitmap rows (a multiple of 128), [4] rows with offsets
-// outside [0,nnz] or descending (also counted in [1]).
-enum { kWDenseAny = 0, kWBad = 1, kWDenseOv = 2, kWDenseHubs = 3, kWBadRows = 4, kWords = 8 };
+// outside [0,nnz] or descending (also counted in [1]), [5] rows i with dense
+// pairs (the length of drows).
+enum { kWDenseAny = 0, kWBad = 1, kWDenseOv = 2, kWDenseHubs = 3, kWBadRows = 4, kWDenseRows = 5, kWords = 8 };
 
 // A nonzero (i, j) at position p of row i is a dense pair when j has a
-// column bitmap (j < hubs) and its prefix row_i[0,p) is longer than the
+// column bitmap (j < hubs) and its prefix row_i[0,p) is longer than 3/8 of the
 // bitmap's ceil(j/32) words plus the margin ov: then one AND and popcount
 // per word of [0,j) costs less than p probes.  Dense pairs get no record;
-// wedge_dense_kernel counts them.
+// wedge_dense_kernel counts them.  At R-MAT scale 22 a margin of 16 takes
+// 4580 us a call with 3/8 of the words, 4640 with half, 4570 with a quarter,
+// about 4850 with all of them and a margin of 32.
 __device__ __forceinline__ bool dense_pair(uint32_t j, uint32_t p, int64_t ov, uint32_t hubs) {
-  return ov >= 0 && j < hubs && static_cast<int64_t>(p) > static_cast<int64_t>((j + 31u) >> 5) + ov;
+  return ov >= 0 && j < hubs && static_cast<int64_t>(p) > static_cast<int64_t>(((j + 31u) >> 5) * 3u >> 3) + ov;
 }
 
 struct Layout {
-  size_t col32, rows16, nlow, in_cnt, in_off, bsum, in_rec, hubs, bits, starts, words, total;
+  size_t col32, rows16, nlow, in_cnt, in_off, bsum, in_rec, hubs, bits, drows, dflag, starts, words, total;
   size_t nvec16;        // 16-byte vectors of rows16, the last one pads
   uint32_t dense_hubs;  // rows with a column bitmap: min(kDenseHubs, numrows rounded up to 128)
   uint32_t chunk;       // nonzeros per chunk of the scan and the fill (a multiple of a warp's round)
@@ -162,6 +167,8 @@ Layout layout(int64_t n, int64_t nnz) {
   // a multiple of 128, so each row's bitmap starts on a 16-byte boundary
   l.dense_hubs = static_cast<uint32_t>(std::min<int64_t>(kDenseHubs, (n + 127) / 128 * 128));
   l.bits = o;   o += up256(static_cast<size_t>(l.dense_hubs) * (l.dense_hubs / 32) * 4);
+  l.drows = o;  o += up256(static_cast<size_t>(n) * 4);
+  l.dflag = o;  o += up256(static_cast<size_t>(n));
   l.starts = o; o += up256(static_cast<size_t>(l.nchunks) * 4);
   l.words = o;  o += up256(kWords * 8);
   l.total = o;
@@ -218,6 +225,7 @@ __device__ __forceinline__ uint64_t vec16(uint32_t b, int64_t i) {
 // Row offsets: rows outside [0,nnz] or descending are counted (the later
 // kernels then return before they use any), the incoming counts are zeroed,
 // nlow[i] (the place of row i's first column that is not low) is set to none,
+// dflag[i] (has row i a dense pair) to no,
 // and starts[c] becomes the row that holds nonzero c * chunk -- so the scan
 // and the fill can split the nonzeros evenly, whatever the rows' lengths.
 // Chunks before the first row's start begin at row 0, those past the last
@@ -225,7 +233,7 @@ __device__ __forceinline__ uint64_t vec16(uint32_t b, int64_t i) {
 __global__ void __launch_bounds__(kRowsThreads)
     wedge_rows_kernel(const int64_t *__restrict__ off, int64_t n, int64_t nnz, uint32_t *__restrict__ in_cnt,
                       uint32_t *__restrict__ nlow, uint4 *__restrict__ rows16, uint64_t nvec16, uint32_t pad,
-                      uint32_t *__restrict__ starts, uint32_t chunk, uint32_t nchunks,
+                      uint8_t *__restrict__ dflag, uint32_t *__restrict__ starts, uint32_t chunk, uint32_t nchunks,
                       unsigned long long *__restrict__ words, unsigned long long *__restrict__ bad,
                       const unsigned *__restrict__ run_if) {
   if (tri::skipped(run_if, 1u)) return;
@@ -236,6 +244,7 @@ __global__ void __launch_bounds__(kRowsThreads)
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * kRowsThreads + threadIdx.x; i < n; i += stride) {
     in_cnt[i] = 0;
     nlow[i] = 0xffffffffu;
+    dflag[i] = 0;
     const int64_t b = off[i], e = off[i + 1];
     if (b < 0 || e < b || e > nnz) {
       nbad++;
@@ -396,8 +405,9 @@ __global__ void __launch_bounds__(kScanThreads, kScanBlocksPerSm)
     wedge_scan_kernel(const int64_t *__restrict__ off, const int64_t *__restrict__ col, int64_t n, int64_t nnz,
                       const uint32_t *__restrict__ starts, uint32_t chunk, uint32_t nchunks,
                       uint32_t *__restrict__ col32, uint16_t *__restrict__ rows16, uint32_t pad,
-                      uint32_t *__restrict__ nlow, uint32_t *__restrict__ in_cnt, uint32_t *__restrict__ hubs,
-                      unsigned long long *__restrict__ words, unsigned long long *__restrict__ bad, int64_t ov,
+                      uint32_t *__restrict__ nlow, uint8_t *__restrict__ dflag, uint32_t *__restrict__ in_cnt,
+                      uint32_t *__restrict__ hubs, unsigned long long *__restrict__ words,
+                      unsigned long long *__restrict__ bad, int64_t ov,
                       uint32_t dhubs, const unsigned *__restrict__ run_if) {
   if (tri::skipped(run_if, 1u)) return;
   if (words[kWBadRows]) return;
@@ -449,6 +459,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanBlocksPerSm)
           const bool inner = in && ok && p[u] > 0;
           const bool dense = inner && dense_pair(cu[u], p[u], ov, dhubs);
           any_dense |= dense;
+          if (dense) dflag[i] = 1;
           count_shared(&hub[cu[u] & (kHub - 1)], inner && !dense && cu[u] < static_cast<uint32_t>(kHub));
           count_global(in_cnt + cu[u], inner && !dense && cu[u] >= static_cast<uint32_t>(kHub));
         }
@@ -1024,11 +1035,12 @@ __global__ void __launch_bounds__(kWarpThreads, kFarBlocksPerSm)
 // Column bitmaps of the rows j below dhubs (their columns all lie in
 // [0, j)), built when the scan met a dense pair: row j's at bits + j *
 // (dhubs / 32), its words zeroed up to a multiple of 4 past ceil(j/32) (the
-// dense kernel reads 16-byte vectors) before its bits are set.
+// dense kernel reads 16-byte vectors) before its bits are set.  And drows, the
+// rows i that have dense pairs.
 __global__ void __launch_bounds__(256)
     wedge_hubbits_kernel(const int64_t *__restrict__ off, const uint32_t *__restrict__ col32, int64_t n,
-                         uint32_t *__restrict__ bits, const unsigned long long *__restrict__ words,
-                         const unsigned *__restrict__ run_if) {
+                         const uint8_t *__restrict__ dflag, uint32_t *__restrict__ drows, uint32_t *__restrict__ bits,
+                         unsigned long long *__restrict__ words, const unsigned *__restrict__ run_if) {
   if (tri::skipped(run_if, 1u)) return;
   if (words[kWBad] || !words[kWDenseAny] || static_cast<int64_t>(words[kWDenseOv]) < 0) return;
   const uint32_t dhubs = static_cast<uint32_t>(words[kWDenseHubs]);
@@ -1036,7 +1048,8 @@ __global__ void __launch_bounds__(256)
   const unsigned lane = lane_id();
   const int64_t rows = static_cast<int64_t>(dhubs) < n ? static_cast<int64_t>(dhubs) : n;
   const int64_t warps = static_cast<int64_t>(gridDim.x) * 8;
-  for (int64_t j = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5); j < rows; j += warps) {
+  const int64_t warp = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  for (int64_t j = warp; j < rows; j += warps) {
     uint32_t *row = bits + static_cast<size_t>(j) * stride;
     const uint32_t nz = ((((static_cast<uint32_t>(j) + 31u) >> 5) + 3u) >> 2) << 2;
     for (uint32_t w = lane; w < nz; w += 32) row[w] = 0;
@@ -1046,59 +1059,75 @@ __global__ void __launch_bounds__(256)
       if (c < static_cast<uint32_t>(j)) atomicOr(&row[c >> 5], 1u << (c & 31));  // the scan checked c < j
     }
   }
+  for (int64_t i0 = warp * 32; i0 < n; i0 += warps * 32) {
+    const bool has = i0 + lane < n && dflag[i0 + lane];
+    const unsigned m = __ballot_sync(kFull, has);
+    if (!m) continue;
+    uint32_t at = 0;
+    if (lane == 0) at = static_cast<uint32_t>(atomicAdd(words + kWDenseRows, 0ull + __popc(m)));
+    at = __shfl_sync(kFull, at, 0) + __popc(m & ((1u << lane) - 1u));
+    if (has) drows[at] = static_cast<uint32_t>(i0 + lane);
+  }
 }
 
-// The dense pairs: one warp per row i that has any, with row i's columns
-// below its largest dense j as bits in the warp's shared memory.  Each pair
+// The dense pairs: a warp claims the rows i that have any, one at a time, with
+// row i's columns below dhubs as bits in the warp's shared memory.  Each pair
 // (i, j) adds popc(row_i & row_j) over the ceil(j/32) words of [0, j) --
 // row j's bits all lie below j.  The 16-byte vectors of up to 32 pairs are
 // flattened over the lanes, kDenseInFlight of them per lane in flight, so a
 // pair costs no round trip of its own.  As the probe kernel would have, each
-// pair adds p to the work tally when row j has columns.
+// pair adds p to the work tally when row j has columns.  (Every warp walking
+// its share of all rows, with a pass over each to see whether it has dense
+// pairs, took 1066 us at R-MAT scale 22 for what the list and claims do in
+// 587: 35 K of 4.2 M rows have any.  5 blocks an SM with 3 vectors in flight
+// 590, 6 with 2 611; carry-save adders before the popcounts 618.)
 constexpr int kDenseInFlight = 4;
 
-__global__ void __launch_bounds__(kDenseThreads)
-    wedge_dense_kernel(const int64_t *__restrict__ off, const uint32_t *__restrict__ col32, int64_t n,
-                       const uint32_t *__restrict__ bits, const unsigned long long *__restrict__ words,
-                       unsigned long long *__restrict__ count, unsigned long long *__restrict__ work,
+__global__ void __launch_bounds__(kDenseThreads, kDenseBlocksPerSm)
+    wedge_dense_kernel(const int64_t *__restrict__ off, const uint32_t *__restrict__ col32,
+                       const uint32_t *__restrict__ drows, const uint32_t *__restrict__ bits,
+                       const unsigned long long *__restrict__ words, unsigned long long *__restrict__ count,
+                       unsigned long long *__restrict__ work, unsigned long long *__restrict__ cursor,
                        const unsigned *__restrict__ run_if) {
   if (tri::skipped(run_if, 1u)) return;
   if (words[kWBad] || !words[kWDenseAny]) return;
   const int64_t ov = static_cast<int64_t>(words[kWDenseOv]);
   const uint32_t dhubs = static_cast<uint32_t>(words[kWDenseHubs]);
   if (ov < 0 || dhubs == 0) return;
-  __shared__ __align__(16) uint32_t bmall[kDenseThreads / 32][kDenseHubs / 32];
-  __shared__ uint32_t stage[kDenseThreads / 32][32];
+  // the vector behind a bitmap stays zero: lanes without a vector read it
+  __shared__ __align__(16) uint32_t bmall[kDenseWarps][kDenseHubs / 32 + 4];
+  __shared__ uint32_t stage[kDenseWarps][32];
   const unsigned lane = lane_id();
   uint32_t *bm = bmall[threadIdx.x >> 5];
   uint32_t *stg = stage[threadIdx.x >> 5];
-  for (int w = lane; w < kDenseHubs / 32; w += 32) bm[w] = 0;
+  for (int w = lane; w < kDenseHubs / 32 + 4; w += 32) bm[w] = 0;
   __syncwarp();
-  const uint32_t stride = dhubs / 32;
+  const uint4 *bm4 = reinterpret_cast<const uint4 *>(bm);
+  const uint4 *bits4 = reinterpret_cast<const uint4 *>(bits);
+  const uint32_t stride4 = dhubs / 128;
+  const unsigned long long nrows = words[kWDenseRows];
   unsigned long long cnt = 0, wk = 0;
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * (kDenseThreads / 32);
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * (kDenseThreads / 32) + (threadIdx.x >> 5); i < n; i += warps) {
-    const int64_t b = off[i], d = off[i + 1] - b;
-    if (d < ov + 2) continue;  // p <= d - 1 must exceed ov + 1
-    uint32_t jmax = 0;
-    for (int64_t k = lane; k < d; k += 32) {
-      const uint32_t c = col32[b + k];
-      if (dense_pair(c, static_cast<uint32_t>(k), ov, dhubs)) jmax = c > jmax ? c : jmax;
-    }
-    jmax = __reduce_max_sync(kFull, jmax);
-    if (jmax == 0) continue;  // a dense j is at least ov + 2
-    for (int64_t k = lane; k < d; k += 32) {
-      const uint32_t c = col32[b + k];
-      if (c < jmax) atomicOr(&bm[c >> 5], 1u << (c & 31));
+  for (;;) {
+    unsigned long long t = 0;
+    if (lane == 0) t = atomicAdd(cursor, 1ull);
+    t = __shfl_sync(kFull, t, 0);
+    if (t >= nrows) break;
+    const uint32_t i = drows[t];
+    const uint32_t b = static_cast<uint32_t>(off[i]), d = static_cast<uint32_t>(off[i + 1]) - b;
+    uint32_t top = 0;  // the row's columns below dhubs are its first ones
+    for (uint32_t k = 0; k < d && top == k; k += 32) {
+      const uint32_t c = k + lane < d ? col32[b + k + lane] : kBadCol;
+      if (c < dhubs) atomicOr(&bm[c >> 5], 1u << (c & 31));
+      top += __popc(__ballot_sync(kFull, c < dhubs));
     }
     __syncwarp();
-    for (int64_t k0 = 0; k0 < d; k0 += 32) {
-      const int64_t k = k0 + lane;
-      const uint32_t c = k < d ? col32[b + k] : kBadCol;
-      const bool dn = k < d && dense_pair(c, static_cast<uint32_t>(k), ov, dhubs);
-      if (dn && off[c + 1] > off[c]) wk += static_cast<unsigned long long>(k);
+    for (uint32_t k0 = 0; k0 < top; k0 += 32) {
+      const uint32_t k = k0 + lane;
+      const uint32_t c = k < top ? col32[b + k] : kBadCol;
+      const bool dn = k < top && dense_pair(c, k, ov, dhubs);
       const unsigned m = __ballot_sync(kFull, dn);
       if (!m) continue;
+      if (dn && off[c + 1] > off[c]) wk += k;
       // the dense columns to the low lanes, so their vector counts strictly increase
       if (dn) stg[__popc(m & ((1u << lane) - 1u))] = c;
       __syncwarp();
@@ -1110,39 +1139,29 @@ __global__ void __launch_bounds__(kDenseThreads)
       const uint32_t nv = lane < nd ? (((cj + 31u) >> 5) + 3u) >> 2 : 0u;
       const uint32_t inc = incl_scan_u32(nv);
       const uint32_t tot = __shfl_sync(kFull, inc, 31);
-      const uint4 *bm4 = reinterpret_cast<const uint4 *>(bm);
-      const uint4 *bits4 = reinterpret_cast<const uint4 *>(bits);
-      const uint32_t stride4 = stride >> 2;
+      const uint32_t q = cj * stride4;  // below 2^21
       uint32_t sum = 0;  // at most 32 pairs of at most 2^14 common columns each
       for (uint32_t base = 0; base < tot; base += 32u * kDenseInFlight) {
         uint4 x[kDenseInFlight], y[kDenseInFlight];
-        bool act[kDenseInFlight];
 #pragma unroll
         for (int h = 0; h < kDenseInFlight; h++) {
           const uint32_t bb = base + 32u * h;
           const int o = flat_owner(inc, bb);
-          const uint32_t j = __shfl_sync(kFull, cj, o);
           const uint32_t v = bb + lane - __shfl_sync(kFull, inc - nv, o);
-          act[h] = bb + lane < tot;
-          // an idle lane reads vector 0 of row j, and its sum is dropped
-          const uint32_t va = act[h] ? v : 0u;
-          x[h] = bits4[static_cast<size_t>(j) * stride4 + va];
-          y[h] = bm4[va];
+          const uint32_t qj = __shfl_sync(kFull, q, o);
+          const bool act = bb + lane < tot;
+          x[h] = bits4[act ? qj + v : 0u];
+          y[h] = bm4[act ? v : kDenseHubs / 128];
         }
 #pragma unroll
-        for (int h = 0; h < kDenseInFlight; h++) {
-          const uint32_t t = __popc(x[h].x & y[h].x) + __popc(x[h].y & y[h].y) + __popc(x[h].z & y[h].z) +
-                             __popc(x[h].w & y[h].w);
-          sum += act[h] ? t : 0u;
-        }
+        for (int h = 0; h < kDenseInFlight; h++)
+          sum += __popc(x[h].x & y[h].x) + __popc(x[h].y & y[h].y) + __popc(x[h].z & y[h].z) +
+                 __popc(x[h].w & y[h].w);
       }
       cnt += sum;
     }
     __syncwarp();
-    for (int64_t k = lane; k < d; k += 32) {
-      const uint32_t c = col32[b + k];
-      if (c < jmax) bm[c >> 5] = 0;
-    }
+    for (uint32_t k = lane; k < top; k += 32) bm[col32[b + k] >> 5] = 0;
     __syncwarp();
   }
   flush(cnt, wk, count, work);
@@ -1172,23 +1191,24 @@ int tri_wedge_prepare(const int64_t *offset, const int64_t *nonzero, int64_t num
   unsigned long long *words = reinterpret_cast<unsigned long long *>(p + l.words);
   uint32_t *starts = reinterpret_cast<uint32_t *>(p + l.starts);
   uint32_t *nlow = reinterpret_cast<uint32_t *>(p + l.nlow);
+  uint8_t *dflag = reinterpret_cast<uint8_t *>(p + l.dflag);
   const uint32_t pad = (1u << warp_bits(numrows)) - 1u;
   // dense pairs (tri.dense 0: none) and their margin over the bitmap's words
-  const int64_t ov = knob_or("tri.dense", 1) == 0 ? -1 : knob_or("tri.dense_ov", 32);
+  const int64_t ov = knob_or("tri.dense", 1) == 0 ? -1 : knob_or("tri.dense_ov", 16);
   BALE_CUDA_OK(cudaMemsetAsync(words, 0, kWords * sizeof(unsigned long long), stream));
   const int64_t rblocks = std::min<int64_t>((numrows + kRowsThreads - 1) / kRowsThreads,
                                             static_cast<int64_t>(num_sms()) * kRowsBlocksPerSm);
   wedge_rows_kernel<<<static_cast<unsigned>(rblocks), kRowsThreads, 0, stream>>>(
-      offset, numrows, nnz, in_cnt, nlow, reinterpret_cast<uint4 *>(p + l.rows16), l.nvec16, pad, starts, l.chunk,
-      l.nchunks, words, bad, run_if);
+      offset, numrows, nnz, in_cnt, nlow, reinterpret_cast<uint4 *>(p + l.rows16), l.nvec16, pad, dflag, starts,
+      l.chunk, l.nchunks, words, bad, run_if);
   BALE_CUDA_OK(cudaGetLastError());
   wedge_scan_kernel<<<l.blocks, kScanThreads, 0, stream>>>(
       offset, nonzero, numrows, nnz, starts, l.chunk, l.nchunks, col32, reinterpret_cast<uint16_t *>(p + l.rows16), pad,
-      nlow, in_cnt, hubs, words, bad, ov, l.dense_hubs, run_if);
+      nlow, dflag, in_cnt, hubs, words, bad, ov, l.dense_hubs, run_if);
   BALE_CUDA_OK(cudaGetLastError());
   if (ov >= 0 && l.dense_hubs > 0) {
-    wedge_hubbits_kernel<<<static_cast<unsigned>((l.dense_hubs + 7) / 8), 256, 0, stream>>>(offset, col32, numrows,
-                                                                                            bits, words, run_if);
+    wedge_hubbits_kernel<<<static_cast<unsigned>((l.dense_hubs + 7) / 8), 256, 0, stream>>>(
+        offset, col32, numrows, dflag, reinterpret_cast<uint32_t *>(p + l.drows), bits, words, run_if);
     BALE_CUDA_OK(cudaGetLastError());
   }
   const int64_t hlim = std::min<int64_t>(kHub, numrows);
@@ -1228,7 +1248,7 @@ int tri_wedge_run(const int64_t *offset, const void *ws, int64_t numrows, int64_
     return static_cast<unsigned>(std::max<int64_t>(
         1, std::min<int64_t>((claims + kWarpWarps - 1) / kWarpWarps, static_cast<int64_t>(sms) * per_sm)));
   };
-  BALE_CUDA_OK(cudaMemsetAsync(cursor, 0, 2 * sizeof(unsigned long long), stream));
+  BALE_CUDA_OK(cudaMemsetAsync(cursor, 0, 3 * sizeof(unsigned long long), stream));
   const int wb = warp_bits(numrows);
   const auto near_kernel = wide ? wedge_near_kernel<true> : wedge_near_kernel<false>;
   near_kernel<<<warps_for(nnz + near * kNearWeight, kNearBlocksPerSm), kWarpThreads,
@@ -1249,9 +1269,10 @@ int tri_wedge_run(const int64_t *offset, const void *ws, int64_t numrows, int64_
   }
   // the dense pairs the prepare step left out of the records (none when its
   // margin was negative: the kernel returns at once)
-  const int64_t dgroups = (numrows + kDenseThreads / 32 - 1) / (kDenseThreads / 32);
-  wedge_dense_kernel<<<static_cast<unsigned>(std::min<int64_t>(dgroups, static_cast<int64_t>(sms) * 8)), kDenseThreads,
-                       0, stream>>>(offset, col32, numrows, bits, words, count, work, run_if);
+  const int64_t dblocks = (numrows + kDenseWarps - 1) / kDenseWarps;
+  wedge_dense_kernel<<<static_cast<unsigned>(std::min<int64_t>(dblocks, static_cast<int64_t>(sms) * kDenseBlocksPerSm)),
+                       kDenseThreads, 0, stream>>>(offset, col32, reinterpret_cast<const uint32_t *>(p + l.drows), bits,
+                                                   words, count, work, cursor + 2, run_if);
   BALE_CUDA_OK(cudaGetLastError());
   return BALE_OK;
 }

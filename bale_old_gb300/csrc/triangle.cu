@@ -239,7 +239,7 @@ int launch_triangle(const int64_t *offset, const int64_t *nonzero, int64_t numro
     // one workspace
     void *ws = device_workspace(
         std::max(tri_wedge_workspace_bytes(numrows, nnz), tri_hybrid_workspace_bytes(numrows, nnz)), stream);
-    unsigned long long *cursor = next_cursor_words(2), *hwords = next_cursor_words(4), *cw = next_cursor_words(4);
+    unsigned long long *cursor = next_cursor_words(3), *hwords = next_cursor_words(4), *cw = next_cursor_words(4);
     if (!ws || !cursor || !hwords || !cw) return BALE_ENOMEM;
     unsigned *choice = reinterpret_cast<unsigned *>(cw + 3);
     BALE_CUDA_OK(cudaMemsetAsync(cw, 0, 3 * sizeof(unsigned long long), stream));
@@ -259,7 +259,7 @@ int launch_triangle(const int64_t *offset, const int64_t *nonzero, int64_t numro
   }
   if ((mode < 0 || mode == 2) && tri_wedge_supported(numrows, nnz)) {
     void *ws = device_workspace(tri_wedge_workspace_bytes(numrows, nnz), stream);
-    unsigned long long *cursor = next_cursor_words(2);
+    unsigned long long *cursor = next_cursor_words(3);
     if (!ws || !cursor) return BALE_ENOMEM;
     return launch_triangle_wedge(offset, nonzero, numrows, nnz, count, work, bad, ws, cursor, stream);
   }

@@ -31,17 +31,20 @@
 //      barrier is ever needed); the warp tests every element of the incoming
 //      prefixes, one shared-memory load each, then clears the bits it set.
 //      Near rows have low columns only, and on a degree-ordered matrix they
-//      are the hubs, where most probes land (80% at R-MAT scale 22); a far
-//      row's other columns are a short sorted list behind a filter.
+//      are the hubs, where most probes land (80% at R-MAT scale 22); far rows
+//      have 2 KiB more for the codes of their other columns, whose few hits
+//      are looked up in the row.
 //      The prefixes are read from a copy of the rows in 16 bits, each row on
 //      a 16-byte boundary and padded so that whole vectors are probed without
 //      a test of where they end: 8 elements and 75 instructions per vector and
 //      lane instead of 4 and 108, half the bytes.  Warps claim equal shares of
 //      the records, not rows: a hub's 54 K prefixes took one warp 2.3 ms.
-//      R-MAT scale 22: 3980 us with 32-bit rows, a 2^16-bit bitmap per
-//      warp (24 warps an SM) and a claim per row; 2806 with 16-bit rows; 2500
-//      as it is, near (40 warps an SM, its shared-memory data pipe 91% busy)
-//      1330 us and far (32 warps, waiting for dependent loads) 1170.
+//      R-MAT scale 22, without the dense pairs of step 5:
+//      3980 us with 32-bit rows, a 2^16-bit bitmap per warp (24 warps an SM)
+//      and a claim per row; 2806 with 16-bit rows; 1850 as it is, near (40
+//      warps an SM, its shared-memory data pipe 91% busy) 970 and far (32
+//      warps) 880, where searching the high part of every prefix in a list of
+//      row j's high columns took 1163.
 //   5. dense pairs: a pair (i,j) whose prefix is long against the ceil(j/32)
 //      words of a bitmap of [0,j) (dense_pair below), for j below 2^14, gets no
 //      record in steps 1-3; step 1 also builds the column bitmaps of the rows
@@ -76,9 +79,11 @@ constexpr int kWarpWarps = kWarpThreads / 32;
 constexpr int kNearBits = 15;
 constexpr uint32_t kNear = 1u << kNearBits;  // rows j below it are near: all their columns are low
 constexpr uint32_t kLow = kNear - 1;         // labels below it are low: bits of a bitmap, values of rows16
-constexpr int kTail = 128;                   // columns of a far row that are not low in shared memory
-constexpr int kFilterWords = 128;            // bits of the filter of those columns, in words
-constexpr int kFarWords = kNear / 32 + kFilterWords + kTail;  // a warp's shared memory in the far kernel
+constexpr uint32_t kHigh = kNear;            // the other labels read as kHigh + their last kHighBits bits
+constexpr int kHighBits = 14;
+constexpr int kTail = 128;                   // high columns of a far row in shared memory
+constexpr uint32_t kFarBits = kHigh + (1u << kHighBits);
+constexpr int kFarWords = kFarBits / 32 + kTail;  // a warp's shared memory in the far kernel
 // A warp claims kSegment units of work, a record being one.  A near row adds
 // kNearWeight (setting and clearing its bitmap: records alone took a graph of
 // 2^14 rows 2x as long, 256 the mixed batch 3% longer), a far row kRowWeight
@@ -87,12 +92,12 @@ constexpr uint32_t kSegment = 512;
 constexpr int kNearWeight = 128;
 constexpr int kRowWeight = 4;
 // Blocks an SM and 16-byte vectors per lane in flight when probing (near:
-// 6 and 2 1470 us, 4 and 4 1375, 5 and 3 1336; far: 5 and 2 spill, 1420 us,
-// 4 and 2 1195, 4 and 3 1167).
+// 6 and 2 1470 us, 4 and 4 1375, 5 and 3 1336; far: 4 and 3 898 us, 4 and 2
+// 878, 3 and 4 in an earlier form 20% more).
 constexpr int kNearBlocksPerSm = 5;
 constexpr int kNearInFlight = 3;
 constexpr int kFarBlocksPerSm = 4;
-constexpr int kFarInFlight = 3;
+constexpr int kFarInFlight = 2;
 constexpr int kUnroll = 2;        // the scan's rounds of 32 nonzeros in flight per warp (4 spill: 510 against 375 us)
 constexpr int kHub = 8192;        // labels whose incoming counts and slots live in shared memory
 constexpr int kScanBlocksPerSm = 3;
@@ -124,7 +129,7 @@ __device__ __forceinline__ bool dense_pair(uint32_t j, uint32_t p, int64_t ov, u
 }
 
 struct Layout {
-  size_t col32, rows16, nlow, in_cnt, in_off, bsum, in_rec, hubs, bits, drows, dflag, starts, words, total;
+  size_t col32, rows16, in_cnt, in_off, bsum, in_rec, hubs, bits, drows, dflag, starts, words, total;
   size_t nvec16;        // 16-byte vectors of rows16, the last one pads
   uint32_t dense_hubs;  // rows with a column bitmap: min(kDenseHubs, numrows rounded up to 128)
   uint32_t chunk;       // nonzeros per chunk of the scan and the fill (a multiple of a warp's round)
@@ -149,7 +154,6 @@ Layout layout(int64_t n, int64_t nnz) {
   l.col32 = o;  o += up256(nz * 4);
   l.nvec16 = nz / 8 + static_cast<size_t>(n) + 1;
   l.rows16 = o; o += up256(l.nvec16 * 16);
-  l.nlow = o;   o += up256(static_cast<size_t>(n) * 4);
   l.in_cnt = o; o += up256(static_cast<size_t>(n) * 4 + 4);
   l.in_off = o; o += up256(static_cast<size_t>(n + 1) * 4);
   l.bsum = o;   o += up256(nb * 4);
@@ -213,18 +217,22 @@ __device__ __forceinline__ int flat_owner(uint32_t inc, uint32_t bb) {
 // rows16 holds the rows' columns as 16 bits each, every row from a 16-byte
 // vector of its own on, row i (which starts at nonzero b) from vector
 // b / 8 + i: a row of d columns needs at most d / 8 + 1 of them, and the next
-// row's start is that far on.  Columns that are not low read as `pad`, and so
-// do the places behind a row's end in its last vector.  No bitmap has the
-// pad's bit set (row j's columns lie below j, and low rows' below the pad's
-// label), and the columns of row i from j on are not in row j either: whole
-// vectors are probed, with no test of where the prefix or the row ends.
+// row's start is that far on.  A low column is itself, a high one a code for
+// 2^18 of them (a hit of which is looked up in the list of row j's high
+// columns); the places behind a row's end in its last vector are pads.  No
+// bitmap has the pad's bit set: row j's columns lie below j, and low ones
+// below the pad.  The columns of row i from j on are not in row j either, so
+// whole vectors are probed with no test of where the prefix or the row ends.
+__device__ __forceinline__ uint32_t code16(uint32_t c) {
+  return c < kLow ? c : kHigh | (c & ((1u << kHighBits) - 1u));
+}
+
 __device__ __forceinline__ uint64_t vec16(uint32_t b, int64_t i) {
   return static_cast<uint64_t>(b >> 3) + static_cast<uint64_t>(i);
 }
 
 // Row offsets: rows outside [0,nnz] or descending are counted (the later
 // kernels then return before they use any), the incoming counts are zeroed,
-// nlow[i] (the place of row i's first column that is not low) is set to none,
 // dflag[i] (has row i a dense pair) to no,
 // and starts[c] becomes the row that holds nonzero c * chunk -- so the scan
 // and the fill can split the nonzeros evenly, whatever the rows' lengths.
@@ -232,7 +240,7 @@ __device__ __forceinline__ uint64_t vec16(uint32_t b, int64_t i) {
 // row's end at row n (no rows).
 __global__ void __launch_bounds__(kRowsThreads)
     wedge_rows_kernel(const int64_t *__restrict__ off, int64_t n, int64_t nnz, uint32_t *__restrict__ in_cnt,
-                      uint32_t *__restrict__ nlow, uint4 *__restrict__ rows16, uint64_t nvec16, uint32_t pad,
+                      uint4 *__restrict__ rows16, uint64_t nvec16, uint32_t pad,
                       uint8_t *__restrict__ dflag, uint32_t *__restrict__ starts, uint32_t chunk, uint32_t nchunks,
                       unsigned long long *__restrict__ words, unsigned long long *__restrict__ bad,
                       const unsigned *__restrict__ run_if) {
@@ -243,7 +251,6 @@ __global__ void __launch_bounds__(kRowsThreads)
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kRowsThreads;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * kRowsThreads + threadIdx.x; i < n; i += stride) {
     in_cnt[i] = 0;
-    nlow[i] = 0xffffffffu;
     dflag[i] = 0;
     const int64_t b = off[i], e = off[i + 1];
     if (b < 0 || e < b || e > nnz) {
@@ -253,7 +260,7 @@ __global__ void __launch_bounds__(kRowsThreads)
     // nnz < 2^32 - 256, so offsets and chunk starts fit 32 bits
     const uint32_t b32 = static_cast<uint32_t>(b), e32 = static_cast<uint32_t>(e);
     // the scan fills in the last vector's columns
-    if (e32 - b32 > 1) rows16[vec16(b32, i) + (e32 - b32 - 1) / 8] = make_uint4(pads, pads, pads, pads);
+    if (e32 > b32) rows16[vec16(b32, i) + (e32 - b32 - 1) / 8] = make_uint4(pads, pads, pads, pads);
     uint32_t c = b32 / chunk + (b32 % chunk ? 1u : 0u);
     if (i == 0)
       for (uint32_t t = 0; t < c && t < nchunks; t++) starts[t] = 0;
@@ -404,8 +411,8 @@ __device__ __forceinline__ uint32_t take_global(uint32_t *a, bool on) {
 __global__ void __launch_bounds__(kScanThreads, kScanBlocksPerSm)
     wedge_scan_kernel(const int64_t *__restrict__ off, const int64_t *__restrict__ col, int64_t n, int64_t nnz,
                       const uint32_t *__restrict__ starts, uint32_t chunk, uint32_t nchunks,
-                      uint32_t *__restrict__ col32, uint16_t *__restrict__ rows16, uint32_t pad,
-                      uint32_t *__restrict__ nlow, uint8_t *__restrict__ dflag, uint32_t *__restrict__ in_cnt,
+                      uint32_t *__restrict__ col32, uint16_t *__restrict__ rows16,
+                      uint8_t *__restrict__ dflag, uint32_t *__restrict__ in_cnt,
                       uint32_t *__restrict__ hubs, unsigned long long *__restrict__ words,
                       unsigned long long *__restrict__ bad, int64_t ov,
                       uint32_t dhubs, const unsigned *__restrict__ run_if) {
@@ -452,8 +459,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanBlocksPerSm)
           const bool ok = cu[u] < i && (p[u] == 0 || cu[u] > prv);
           if (in) {
             col32[k[u]] = ok ? cu[u] : kBadCol;
-            rows16[vec16(k[u] - p[u], i) * 8 + p[u]] = static_cast<uint16_t>(cu[u] < pad ? cu[u] : pad);
-            if (cu[u] >= kLow && (p[u] == 0 || prv < kLow)) nlow[i] = p[u];
+            rows16[vec16(k[u] - p[u], i) * 8 + p[u]] = static_cast<uint16_t>(code16(cu[u]));
           }
           nbad += in && !ok;
           const bool inner = in && ok && p[u] > 0;
@@ -667,18 +673,47 @@ __device__ __forceinline__ uint32_t lds(uint32_t a) {
 // a left shift by the label leaves its bit in the sign.
 __device__ __forceinline__ uint32_t low_bit(uint32_t c) { return 0x80000000u >> (c & 31u); }
 
-// cnt + the number of the eight 16-bit labels of x that are set in the
-// bitmap at shared-memory address bm.
-__device__ __forceinline__ uint32_t test8(uint32_t bm, uint4 x, uint32_t cnt) {
-  const uint32_t v[4] = {x.x, x.y, x.z, x.w};
+// cnt + the number of the eight 16-bit codes of x that are set in the
+// bitmap at shared-memory address bm.  FAR: the sign of *high is set when one
+// of them stands for high labels; else those are not looked up (they are
+// columns from j on, and the bitmap ends before them).
+template <bool FAR>
+__device__ __forceinline__ uint32_t test8(uint32_t bm, uint4 x, uint32_t cnt, uint32_t *high) {
+  uint32_t v[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
   for (int t = 0; t < 4; t++) {
+    if (!FAR) v[t] = __vminu2(v[t], kLow * 0x10001u);
     const uint32_t w0 = lds(shr_add<3>(v[t] & 0xffe0u, bm));
     const uint32_t w1 = lds(shr_add<19>(v[t] & 0xffe00000u, bm));
-    cnt = shr_add<31>(__funnelshift_l(0u, w0, v[t]), cnt);
-    cnt = shr_add<31>(__funnelshift_l(0u, w1, v[t] >> 16), cnt);
+    const uint32_t s0 = __funnelshift_l(0u, w0, v[t]), s1 = __funnelshift_l(0u, w1, v[t] >> 16);
+    cnt = shr_add<31>(s0, cnt);
+    cnt = shr_add<31>(s1, cnt);
+    if (FAR) *high |= (s0 & (v[t] << 16)) | (s1 & v[t]);
   }
   return cnt;
+}
+
+// The bits of a row of d columns, which starts at vector v0 of rows16 and
+// whose last vector is filled up with pads, set in or taken out of the bitmap
+// bm of `bits` codes (whole warp): eight columns a load.  Returns the number
+// of low ones in this lane.
+template <bool SET>
+__device__ __forceinline__ uint32_t mark_row(uint32_t *bm, uint32_t bits, const uint4 *__restrict__ rows16,
+                                             uint64_t v0, uint32_t d, uint32_t pad) {
+  uint32_t low = 0;
+  for (uint32_t v = lane_id(); v < (d + 7u) >> 3; v += 32) {
+    const uint4 x = rows16[v0 + v];
+    const uint32_t two[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int t = 0; t < 8; t++) {
+      const uint32_t c = t & 1 ? two[t >> 1] >> 16 : two[t >> 1] & 0xffffu;
+      if (c == pad || c >= bits) continue;
+      if (SET) atomicOr(&bm[c >> 5], low_bit(c));
+      else bm[c >> 5] = 0;
+      low += c < kLow;
+    }
+  }
+  return low;
 }
 
 // Hits in the bitmap at bm among the vectors of nrec prefixes.  fetch(r)
@@ -686,73 +721,53 @@ __device__ __forceinline__ uint32_t test8(uint32_t bm, uint4 x, uint32_t cnt) {
 // 0 in the lanes behind the last prefix).  The vectors of 32 prefixes are
 // flattened over the warp, so every lane has one whatever the prefix lengths,
 // K vectors per lane in flight.  Lanes without a vector read the last one,
-// which is all pads.  WIDE: 2^32 vectors and more.  (Vectors asked for ahead
+// which is all pads.  FAR: check(x, t, o, hit) gives the number of x's codes that
+// were hit for another high label, x being vector t of lane o's prefix; it is
+// called by all lanes, `hit` saying which have such a code.  WIDE: 2^32 vectors and more.  (Vectors asked for ahead
 // across the ends of the batches, one at a time or in pairs: 2806 -> 3180 and
 // 2660 us against 2610, the registers costing more than the waits.)
-template <bool WIDE, int K, class Fetch>
+template <bool WIDE, bool FAR, int K, class Fetch, class Check>
 __device__ __forceinline__ unsigned long long probe_stream(uint32_t bm, const uint4 *__restrict__ rows16,
-                                                           uint64_t nvec16, uint32_t nrec, Fetch fetch) {
+                                                           uint64_t nvec16, uint32_t nrec, Fetch fetch, Check check) {
   using Index = typename std::conditional<WIDE, uint64_t, uint32_t>::type;
   const unsigned lane = lane_id();
   const Index pads = static_cast<Index>(nvec16 - 1);
-  uint32_t r = 0, base = 0, tot = 0, inc = 0;
-  Index q = 0;
-  const auto issue = [&](uint4 *x) -> bool {
-    if (base >= tot) {
-      if (r >= nrec) return false;
-      uint64_t v0 = 0;
-      const uint32_t nv = fetch(r, v0);
-      r += 32;
-      inc = incl_scan_u32(nv);
-      tot = __shfl_sync(kFull, inc, 31);
-      q = static_cast<Index>(v0) - (inc - nv);  // vector index = q + flattened position
-      base = 0;
-    }
-#pragma unroll
-    for (int h = 0; h < K; h++) {
-      const uint32_t bb = base + 32u * h;
-      Index v = __shfl_sync(kFull, q, flat_owner(inc, bb)) + (bb + lane);
-      v = bb + lane < tot && v < pads ? v : pads;
-      x[h] = rows16[v];
-    }
-    base += 32 * K;
-    return true;
-  };
-  const auto test = [&](const uint4 *x) {
-    uint32_t c = 0;
-#pragma unroll
-    for (int h = 0; h < K; h++) c = test8(bm, x[h], c);
-    return c;
-  };
-  uint4 x[K];
   unsigned long long total = 0;
-  while (issue(x)) total += test(x);
-  return total;
-}
-
-// The filter of a far row's columns that are not low: their low 12 bits.
-__device__ __forceinline__ uint32_t filter_word(uint32_t c) { return (c >> 5) & (kFilterWords - 1); }
-
-// The elements of up to 32 runs of columns (lane l holds run [s, s + c), c >= 1
-// but in the lanes behind the last) that are in the ascending list
-// tail[0,ntail), whose columns are set in the filter: whole warp, the runs
-// flattened over the lanes.
-__device__ __forceinline__ uint32_t probe_tail(const uint32_t *filter, const uint32_t *__restrict__ tail,
-                                               uint32_t ntail, const uint32_t *__restrict__ col32, uint32_t s,
-                                               uint32_t c) {
-  const unsigned lane = lane_id();
-  const uint32_t inc = incl_scan_u32(c);
-  const uint32_t tot = __shfl_sync(kFull, inc, 31);
-  const uint32_t q = s - (inc - c);
-  uint32_t cnt = 0;
-  for (uint32_t base = 0; base < tot; base += 32) {
-    const uint32_t k = __shfl_sync(kFull, q, flat_owner(inc, base)) + base + lane;
-    if (base + lane < tot) {
-      const uint32_t w = col32[k];
-      if ((filter[filter_word(w)] & low_bit(w)) && search_u32(tail, ntail, w)) cnt++;
+  for (uint32_t r = 0; r < nrec; r += 32) {
+    uint64_t v0 = 0;
+    const uint32_t nv = fetch(r, v0);
+    const uint32_t inc = incl_scan_u32(nv);
+    const uint32_t tot = __shfl_sync(kFull, inc, 31);
+    const Index q = static_cast<Index>(v0) - (inc - nv);  // vector index = q + flattened position
+    for (uint32_t base = 0; base < tot; base += 32 * K) {
+      uint4 x[K];
+#pragma unroll
+      for (int h = 0; h < K; h++) {
+        const uint32_t bb = base + 32u * h;
+        Index v = __shfl_sync(kFull, q, flat_owner(inc, bb)) + (bb + lane);
+        v = bb + lane < tot && v < pads ? v : pads;
+        x[h] = rows16[v];
+      }
+      uint32_t c = 0, high[K];
+#pragma unroll
+      for (int h = 0; h < K; h++) {
+        high[h] = 0;
+        c = test8<FAR>(bm, x[h], c, &high[h]);
+      }
+      total += c;
+      if (FAR) {
+#pragma unroll
+        for (int h = 0; h < K; h++) {
+          if (!__any_sync(kFull, static_cast<int32_t>(high[h]) < 0)) continue;
+          const uint32_t bb = base + 32u * h;
+          const int o = flat_owner(inc, bb);
+          const uint32_t t = bb + lane - __shfl_sync(kFull, inc - nv, o);
+          total -= check(x[h], t, o, static_cast<int32_t>(high[h]) < 0);
+        }
+      }
     }
   }
-  return cnt;
+  return total;
 }
 
 // Probes of up to 32 prefixes of different rows j (lane l holds record l
@@ -815,9 +830,9 @@ __device__ __forceinline__ void flush(unsigned long long cnt, unsigned long long
 // place(j + 1), its records first; a row may be cut between claims.
 template <bool WIDE>
 __global__ void __launch_bounds__(kWarpThreads, kNearBlocksPerSm)
-    wedge_near_kernel(const int64_t *__restrict__ off, const uint32_t *__restrict__ col32,
-                      const uint4 *__restrict__ rows16, uint64_t nvec16, const uint32_t *__restrict__ in_off,
-                      const uint2 *__restrict__ in_rec, uint32_t rows, int nearbits,
+    wedge_near_kernel(const int64_t *__restrict__ off, const uint4 *__restrict__ rows16, uint64_t nvec16,
+                      const uint32_t *__restrict__ in_off, const uint2 *__restrict__ in_rec, uint32_t rows,
+                      int nearbits,
                       const unsigned long long *__restrict__ words, unsigned long long *__restrict__ count,
                       unsigned long long *__restrict__ work, unsigned long long *__restrict__ cursor,
                       const unsigned *__restrict__ run_if) {
@@ -825,7 +840,7 @@ __global__ void __launch_bounds__(kWarpThreads, kNearBlocksPerSm)
   extern __shared__ uint32_t wsm[];
   if (words[kWBad]) return;
   const unsigned lane = lane_id();
-  const uint32_t nw = 1u << (nearbits - 5);
+  const uint32_t nw = 1u << (nearbits - 5), pad = 32u * nw - 1u;
   uint32_t *bm = wsm + static_cast<size_t>(threadIdx.x >> 5) * nw;
   const uint32_t bma = static_cast<uint32_t>(__cvta_generic_to_shared(bm));
   for (uint32_t w = lane; w < nw; w += 32) bm[w] = 0;
@@ -849,22 +864,21 @@ __global__ void __launch_bounds__(kWarpThreads, kNearBlocksPerSm)
       const uint32_t b = static_cast<uint32_t>(off[j]), d = static_cast<uint32_t>(off[j + 1]) - b;
       if (hi <= lo || d == 0) continue;
       const uint32_t r0 = static_cast<uint32_t>(lo), nrec = static_cast<uint32_t>(hi - lo);
-      for (uint32_t k = lane; k < d; k += 32) {
-        const uint32_t c = col32[b + k];
-        atomicOr(&bm[(c >> 5) & (nw - 1u)], low_bit(c));
-      }
-      __syncwarp();
       uint2 next = lane < nrec ? in_rec[r0 + lane] : make_uint2(0u, 0u);
-      cnt += probe_stream<WIDE, kNearInFlight>(bma, rows16, nvec16, nrec, [&](uint32_t r, uint64_t &v0) {
+      mark_row<true>(bm, 32u * nw, rows16, vec16(b, j), d, pad);
+      __syncwarp();
+      const auto fetch = [&](uint32_t r, uint64_t &v0) {
         const uint2 rec = next;
         next = r + 32 + lane < nrec ? in_rec[r0 + r + 32 + lane] : make_uint2(0u, 0u);
         const uint32_t p = rec.y & 0xffffu;
         v0 = rec.x | (WIDE ? static_cast<uint64_t>(rec.y >> 16) << 32 : uint64_t(0));
         wk += p;
         return (p + 7u) >> 3;
-      });
+      };
+      cnt += probe_stream<WIDE, false, kNearInFlight>(bma, rows16, nvec16, nrec, fetch,
+                                                      [](uint4, uint32_t, int, bool) { return 0u; });
       __syncwarp();
-      for (uint32_t k = lane; k < d; k += 32) bm[(col32[b + k] >> 5) & (nw - 1u)] = 0;
+      mark_row<false>(bm, 32u * nw, rows16, vec16(b, j), d, pad);
       __syncwarp();
     }
   }
@@ -873,13 +887,13 @@ __global__ void __launch_bounds__(kWarpThreads, kNearBlocksPerSm)
 
 // The far rows j, from kNear on, claimed in the same way but looked at 32 at a
 // time, one lane each, so that rows without records cost no serial loads.  A
-// warp has a bitmap of the low labels, the filter of row j's other columns
-// and room for kTail of them.
+// warp has a bitmap of the low labels and the codes of the high ones, and room
+// for kTail high columns of row j.
 template <bool WIDE>
 __global__ void __launch_bounds__(kWarpThreads, kFarBlocksPerSm)
     wedge_far_kernel(const int64_t *__restrict__ off, const uint32_t *__restrict__ col32,
-                     const uint4 *__restrict__ rows16, uint64_t nvec16, const uint32_t *__restrict__ nlow,
-                     const uint32_t *__restrict__ in_off, const uint2 *__restrict__ in_rec, int64_t n,
+                     const uint4 *__restrict__ rows16, uint64_t nvec16, const uint32_t *__restrict__ in_off,
+                     const uint2 *__restrict__ in_rec, int64_t n,
                      uint32_t nvec_all, uint32_t stage_max, const unsigned long long *__restrict__ words,
                      unsigned long long *__restrict__ count, unsigned long long *__restrict__ work,
                      unsigned long long *__restrict__ cursor, const unsigned *__restrict__ run_if) {
@@ -890,11 +904,10 @@ __global__ void __launch_bounds__(kWarpThreads, kFarBlocksPerSm)
   constexpr int64_t near = kNear;
   constexpr uint32_t nw = kNear / 32;
   uint32_t *bm = wsm + static_cast<size_t>(threadIdx.x >> 5) * kFarWords;
-  uint32_t *filter = bm + nw;
-  uint32_t *list = filter + kFilterWords;
+  uint32_t *list = bm + kFarBits / 32;
   const uint32_t bma = static_cast<uint32_t>(__cvta_generic_to_shared(bm));
   const uint4 *__restrict__ col4 = reinterpret_cast<const uint4 *>(col32);  // col32 is 256-byte aligned
-  for (uint32_t w = lane; w < nw + kFilterWords; w += 32) bm[w] = 0;
+  for (uint32_t w = lane; w < kFarBits / 32; w += 32) bm[w] = 0;
   __syncwarp();
   unsigned long long cnt = 0, wk = 0;
   const auto place = [in_off](int64_t j) {
@@ -988,43 +1001,46 @@ __global__ void __launch_bounds__(kWarpThreads, kFarBlocksPerSm)
         todo &= todo - 1;
         const uint32_t r0 = __shfl_sync(kFull, lr0, at), nrec = __shfl_sync(kFull, lnr, at);
         const uint32_t b = __shfl_sync(kFull, lb, at), d = __shfl_sync(kFull, ld, at);
-        uint2 next = lane < nrec ? in_rec[r0 + lane] : make_uint2(0u, 0u);
-        // row j's low columns go to the bitmap, the others (its ascending tail) to the filter
-        uint32_t below = 0;
-        for (uint32_t k = lane; k < d; k += 32) {
-          const uint32_t c = col32[b + k];
-          atomicOr(c < kLow ? &bm[c >> 5] : &filter[filter_word(c)], low_bit(c));
-          below += c < kLow;
+        const int64_t j = j0 - 32 + at;
+        // a record is known two batches ahead and its row's start one
+        uint2 rec = lane < nrec ? in_rec[r0 + lane] : make_uint2(0u, 0u);
+        uint2 next = 32 + lane < nrec ? in_rec[r0 + 32 + lane] : make_uint2(0u, 0u);
+        const uint32_t below = __reduce_add_sync(kFull, mark_row<true>(bm, kFarBits, rows16, vec16(b, j), d, kLow));
+        uint32_t start = rec.y ? static_cast<uint32_t>(off[rec.x]) : 0u, from = 0, len = 0;
+        const uint32_t *high = col32 + b + below;  // row j's high columns
+        const uint32_t nhigh = d - below;
+        if (nhigh <= static_cast<uint32_t>(kTail)) {
+          for (uint32_t k = lane; k < nhigh; k += 32) list[k] = high[k];
+          high = list;
         }
-        below = __reduce_add_sync(kFull, below);
-        const uint32_t ntail = d - below;
-        const bool cached = ntail <= static_cast<uint32_t>(kTail);
-        if (cached)
-          for (uint32_t k = lane; k < ntail; k += 32) list[k] = col32[b + below + k];
         __syncwarp();
-        cnt += probe_stream<WIDE, kFarInFlight>(bma, rows16, nvec16, nrec, [&](uint32_t r, uint64_t &v0) {
-          const uint2 rec = next;
-          next = r + 32 + lane < nrec ? in_rec[r0 + r + 32 + lane] : make_uint2(0u, 0u);
-          const uint32_t p = rec.y;
-          uint32_t start = 0, low = 0;
-          if (p) {
-            start = static_cast<uint32_t>(off[rec.x]);
-            low = nlow[rec.x] < p ? nlow[rec.x] : p;
-          }
+        const auto fetch = [&](uint32_t r, uint64_t &v0) {
+          from = start;
+          len = rec.y;
           v0 = vec16(start, rec.x);
-          wk += p;
-          // a prefix with no high column gives j itself, at place p, which row j does not have
-          const uint32_t high = p ? (p > low ? p - low : 1u) : 0u;
-          if (ntail)
-            cnt += cached ? probe_tail(filter, list, ntail, col32, start + low, high)
-                          : probe_tail(filter, col32 + b + below, ntail, col32, start + low, high);
-          return p ? (low + (low ? 7u : 8u)) >> 3 : 0u;  // with no low column still a vector (of pads)
-        });
+          wk += len;
+          rec = next;
+          start = rec.y ? static_cast<uint32_t>(off[rec.x]) : 0u;
+          next = r + 64 + lane < nrec ? in_rec[r0 + r + 64 + lane] : make_uint2(0u, 0u);
+          return len ? ((len - 1u) >> 3) + 1u : 0u;
+        };
+        const auto check = [&](uint4 x, uint32_t t, int o, bool hit) {
+          const uint32_t s = __shfl_sync(kFull, from, o), p = __shfl_sync(kFull, len, o);
+          uint32_t wrong = 0;
+          if (hit) {
+            const uint32_t two[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+              const uint32_t c = e & 1 ? two[e >> 1] >> 16 : two[e >> 1] & 0xffffu;
+              if (c < kHigh || !(bm[c >> 5] & low_bit(c))) continue;
+              if (8u * t + e >= p || !search_u32(high, nhigh, col32[s + 8u * t + e])) wrong++;
+            }
+          }
+          return wrong;
+        };
+        cnt += probe_stream<WIDE, true, kFarInFlight>(bma, rows16, nvec16, nrec, fetch, check);
         __syncwarp();
-        for (uint32_t k = lane; k < d; k += 32) {
-          const uint32_t c = col32[b + k];
-          *(c < kLow ? &bm[c >> 5] : &filter[filter_word(c)]) = 0;
-        }
+        mark_row<false>(bm, kFarBits, rows16, vec16(b, j), d, kLow);
         __syncwarp();
       }
     }
@@ -1167,6 +1183,8 @@ __global__ void __launch_bounds__(kDenseThreads, kDenseBlocksPerSm)
   flush(cnt, wk, count, work);
 }
 
+bool g_far_attr[2][64];
+
 }  // namespace
 
 bool tri_wedge_supported(int64_t numrows, int64_t nnz) {
@@ -1190,7 +1208,6 @@ int tri_wedge_prepare(const int64_t *offset, const int64_t *nonzero, int64_t num
   uint32_t *bits = reinterpret_cast<uint32_t *>(p + l.bits);
   unsigned long long *words = reinterpret_cast<unsigned long long *>(p + l.words);
   uint32_t *starts = reinterpret_cast<uint32_t *>(p + l.starts);
-  uint32_t *nlow = reinterpret_cast<uint32_t *>(p + l.nlow);
   uint8_t *dflag = reinterpret_cast<uint8_t *>(p + l.dflag);
   const uint32_t pad = (1u << warp_bits(numrows)) - 1u;
   // dense pairs (tri.dense 0: none) and their margin over the bitmap's words
@@ -1199,12 +1216,12 @@ int tri_wedge_prepare(const int64_t *offset, const int64_t *nonzero, int64_t num
   const int64_t rblocks = std::min<int64_t>((numrows + kRowsThreads - 1) / kRowsThreads,
                                             static_cast<int64_t>(num_sms()) * kRowsBlocksPerSm);
   wedge_rows_kernel<<<static_cast<unsigned>(rblocks), kRowsThreads, 0, stream>>>(
-      offset, numrows, nnz, in_cnt, nlow, reinterpret_cast<uint4 *>(p + l.rows16), l.nvec16, pad, dflag, starts,
+      offset, numrows, nnz, in_cnt, reinterpret_cast<uint4 *>(p + l.rows16), l.nvec16, pad, dflag, starts,
       l.chunk, l.nchunks, words, bad, run_if);
   BALE_CUDA_OK(cudaGetLastError());
   wedge_scan_kernel<<<l.blocks, kScanThreads, 0, stream>>>(
-      offset, nonzero, numrows, nnz, starts, l.chunk, l.nchunks, col32, reinterpret_cast<uint16_t *>(p + l.rows16), pad,
-      nlow, dflag, in_cnt, hubs, words, bad, ov, l.dense_hubs, run_if);
+      offset, nonzero, numrows, nnz, starts, l.chunk, l.nchunks, col32, reinterpret_cast<uint16_t *>(p + l.rows16),
+      dflag, in_cnt, hubs, words, bad, ov, l.dense_hubs, run_if);
   BALE_CUDA_OK(cudaGetLastError());
   if (ov >= 0 && l.dense_hubs > 0) {
     wedge_hubbits_kernel<<<static_cast<unsigned>((l.dense_hubs + 7) / 8), 256, 0, stream>>>(
@@ -1253,17 +1270,22 @@ int tri_wedge_run(const int64_t *offset, const void *ws, int64_t numrows, int64_
   const auto near_kernel = wide ? wedge_near_kernel<true> : wedge_near_kernel<false>;
   near_kernel<<<warps_for(nnz + near * kNearWeight, kNearBlocksPerSm), kWarpThreads,
                 (size_t(1) << (wb - 3)) * kWarpWarps, stream>>>(
-      offset, col32, rows16, l.nvec16, in_off, in_rec, static_cast<uint32_t>(near), wb, words, count, work, cursor,
-      run_if);
+      offset, rows16, l.nvec16, in_off, in_rec, static_cast<uint32_t>(near), wb, words, count, work, cursor, run_if);
   BALE_CUDA_OK(cudaGetLastError());
   if (near < numrows) {
     const uint32_t nvec_all = static_cast<uint32_t>((nnz + 3) / 4);
     const uint32_t stage_max =
         static_cast<uint32_t>(std::min<int64_t>(knob_or("tri.wedge_stage_max", 64), kNear / 32));
     const auto far_kernel = wide ? wedge_far_kernel<true> : wedge_far_kernel<false>;
+    const int dev = current_device();
+    if (dev >= 0 && dev < 64 && !g_far_attr[wide][dev]) {
+      BALE_CUDA_OK(cudaFuncSetAttribute(far_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(kFarWords * sizeof(uint32_t) * kWarpWarps)));
+      g_far_attr[wide][dev] = true;
+    }
     far_kernel<<<warps_for(nnz + (numrows - near) * kRowWeight, kFarBlocksPerSm), kWarpThreads,
                  kFarWords * sizeof(uint32_t) * kWarpWarps, stream>>>(
-        offset, col32, rows16, l.nvec16, reinterpret_cast<const uint32_t *>(p + l.nlow), in_off, in_rec, numrows,
+        offset, col32, rows16, l.nvec16, in_off, in_rec, numrows,
         nvec_all, stage_max, words, count, work, cursor + 1, run_if);
     BALE_CUDA_OK(cudaGetLastError());
   }

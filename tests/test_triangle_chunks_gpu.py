@@ -118,3 +118,27 @@ def test_rows_around_the_low_labels(cuda, bale, oracle, wedge, n):
         rows.append(r.astype(np.int64))
         off[i + 1] = off[i] + r.size
     _check(bale, oracle, off, np.concatenate(rows))
+
+
+@pytest.mark.parametrize("many", [3, 40, 200])
+def test_high_labels_that_share_a_code(cuda, bale, oracle, wedge, many):
+    """Columns from 2^15 on that are equal in their last 14 bits: neighbours of
+    one row (as many as the list holds and more), of another row only, or both."""
+    rng = np.random.default_rng(many)
+    base = np.sort(rng.choice(np.arange(32_767, 40_000), many, replace=False))
+    labels = np.unique(np.concatenate([base + 16_384 * k for k in range(4)]))
+    low = np.arange(100, 170)
+    n = 100_600
+    off, rows = np.zeros(n + 1, np.int64), []
+    for i in range(n):
+        if i >= n - 60 or (i in labels and i % 3 == 0):
+            below = labels[labels < i]
+            r = np.union1d(low, rng.choice(below, int(rng.integers(below.size // 2, below.size + 1)), replace=False)) \
+                if below.size else low
+            if i >= n - 60:
+                r = np.union1d(r, np.arange(n - 60, i))
+        else:
+            r = np.zeros(0, np.int64)
+        rows.append(np.asarray(r, np.int64))
+        off[i + 1] = off[i] + rows[-1].size
+    _check(bale, oracle, off, np.concatenate(rows))

@@ -145,14 +145,16 @@ int tri_hybrid_run(const int64_t *offset, const uint32_t *col32, const uint32_t 
 // about 2^32 nonzeros.  prepare builds the u32 column copy and the transpose
 // into ws (tri_wedge_workspace_bytes) and adds malformed entries to *bad (may
 // be NULL); run counts from a prepared ws (cursor: three device words, zeroed
-// there); launch_triangle_wedge does both.
+// there unless `zeroed`, or by prepare when it is given them);
+// launch_triangle_wedge does both.
 bool tri_wedge_supported(int64_t numrows, int64_t nnz);
 size_t tri_wedge_workspace_bytes(int64_t numrows, int64_t nnz);
 int tri_wedge_prepare(const int64_t *offset, const int64_t *nonzero, int64_t numrows, int64_t nnz, void *ws,
-                      unsigned long long *bad, cudaStream_t stream, const unsigned *run_if = nullptr);
+                      unsigned long long *bad, cudaStream_t stream, const unsigned *run_if = nullptr,
+                      unsigned long long *cursor = nullptr);
 int tri_wedge_run(const int64_t *offset, const void *ws, int64_t numrows, int64_t nnz, unsigned long long *count,
                   unsigned long long *work, unsigned long long *cursor, cudaStream_t stream,
-                  const unsigned *run_if = nullptr);
+                  const unsigned *run_if = nullptr, bool zeroed = false);
 int launch_triangle_wedge(const int64_t *offset, const int64_t *nonzero, int64_t numrows, int64_t nnz,
                           unsigned long long *count, unsigned long long *work, unsigned long long *bad, void *ws,
                           unsigned long long *cursor, cudaStream_t stream, const unsigned *run_if = nullptr);

@@ -225,9 +225,9 @@ def tune_batch(quick: bool) -> tuple[dict, list]:
     dev = torch.device("cuda:0")
     rows, knobs = [], {}
     small = build_mix(dev, MIX_SMALL)
-    tiles = (1 << 15, 1 << 16, 1 << 17, 1 << 18)
+    tiles = (1 << 13, 1 << 14, 1 << 15, 1 << 16, 1 << 17)
     plan = [("batch.histo_tile", tiles), ("batch.histo_l2_tile", tiles), ("batch.ig_tile", tiles),
-            ("batch.tri_light_rows", (1 << 13, 1 << 15, 1 << 17)), ("batch.tri_heavy_rows", (1, 4))]
+            ("batch.tri_light_rows", (1 << 12, 1 << 13, 1 << 15, 1 << 17)), ("batch.tri_heavy_rows", (1, 4))]
     for cls in ("small", "medium"):
         for base, cands in plan:
             name = f"{base}.{cls}"

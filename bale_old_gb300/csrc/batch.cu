@@ -13,7 +13,8 @@
 //                                    shared-memory copy of the table, then
 //                                    flushed with one L2 reduction per counter;
 //   histo, larger table            : plain red.global.add.u64 per update;
-//   ig                             : direct gather, 8 loads in flight/thread;
+//   ig                             : direct gather, 8 loads in flight/thread
+//                                    and the next 8 indices behind them;
 //   triangles, light rows          : warps take rows of the task's range
 //                                    (tri_device.cuh light_row);
 //   triangles, heavy rows          : the whole block per heavy row, row i as
@@ -51,15 +52,41 @@ __device__ __forceinline__ void add_bad(unsigned long long *bad, unsigned long l
   if (lane_id() == 0 && v) atomicAdd(bad, v);
 }
 
+// Indices a thread has in flight; the next ones are asked for while it works
+// on these (256 histograms and 192 gathers in one batch: 796 -> 736 us).
+constexpr int kInFlight = 8;
+
+// Calls f(position, index) for the thread's positions of [lo,hi), whose
+// indices are loaded kInFlight at a time, the next ones before f sees these.
+template <class F>
+__device__ __forceinline__ void for_indices(const int64_t *__restrict__ in, int64_t lo, int64_t hi, F f) {
+  int64_t r[kInFlight];
+  const auto load = [&](int64_t i) {
+#pragma unroll
+    for (int u = 0; u < kInFlight; u++) r[u] = (i + u * kThreads < hi) ? ld_stream(in + i + u * kThreads) : 0;
+  };
+  int64_t i = lo + threadIdx.x;
+  load(i);
+  for (; i < hi; i += kInFlight * kThreads) {
+    int64_t now[kInFlight];
+#pragma unroll
+    for (int u = 0; u < kInFlight; u++) now[u] = r[u];
+    load(i + kInFlight * kThreads);
+#pragma unroll
+    for (int u = 0; u < kInFlight; u++)
+      if (i + u * kThreads < hi) f(i + u * kThreads, now[u]);
+  }
+}
+
 __device__ void cta_histo_smem(const Inst &in, int64_t lo, int64_t hi, uint32_t *sm, unsigned long long *bad) {
   const uint64_t m = static_cast<uint64_t>(in.m);
   for (uint64_t c = threadIdx.x; c < m; c += kThreads) sm[c] = 0;
   __syncthreads();
   unsigned long long nb = 0;
-  for (int64_t i = lo + threadIdx.x; i < hi; i += kThreads) {
-    const uint64_t k = static_cast<uint64_t>(ld_stream(in.in + i) >> in.shift);
+  for_indices(in.in, lo, hi, [&](int64_t, int64_t r) {
+    const uint64_t k = static_cast<uint64_t>(r >> in.shift);
     if (k < m) atomicAdd(&sm[k], 1u); else nb++;
-  }
+  });
   __syncthreads();
   for (uint64_t c = threadIdx.x; c < m; c += kThreads) {
     const uint32_t v = sm[c];
@@ -71,29 +98,26 @@ __device__ void cta_histo_smem(const Inst &in, int64_t lo, int64_t hi, uint32_t 
 __device__ void cta_histo_l2(const Inst &in, int64_t lo, int64_t hi, unsigned long long *bad) {
   const uint64_t m = static_cast<uint64_t>(in.m);
   unsigned long long nb = 0;
-  for (int64_t i = lo + threadIdx.x; i < hi; i += 4 * kThreads) {
-    int64_t r[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) r[u] = (i + u * kThreads < hi) ? ld_stream(in.in + i + u * kThreads) : -1;
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      if (i + u * kThreads < hi) {
-        const uint64_t k = static_cast<uint64_t>(r[u] >> in.shift);
-        if (k < m) red_add_u64(in.out + k, 1ull); else nb++;
-      }
-    }
-  }
+  for_indices(in.in, lo, hi, [&](int64_t, int64_t r) {
+    const uint64_t k = static_cast<uint64_t>(r >> in.shift);
+    if (k < m) red_add_u64(in.out + k, 1ull); else nb++;
+  });
   add_bad(bad, nb);
 }
 
 __device__ void cta_ig(const Inst &in, int64_t lo, int64_t hi, unsigned long long *bad) {
   const uint64_t m = static_cast<uint64_t>(in.m);
   unsigned long long nb = 0;
-  constexpr int U = 8;
-  for (int64_t i = lo + threadIdx.x; i < hi; i += U * kThreads) {
-    int64_t r[U], v[U];
+  constexpr int U = kInFlight;
+  int64_t r[U];
+  const auto load = [&](int64_t i) {
 #pragma unroll
     for (int u = 0; u < U; u++) r[u] = (i + u * kThreads < hi) ? ld_stream(in.in + i + u * kThreads) : 0;
+  };
+  int64_t i = lo + threadIdx.x;
+  load(i);
+  for (; i < hi; i += U * kThreads) {
+    int64_t v[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const uint64_t k = static_cast<uint64_t>(r[u] >> in.shift);
@@ -102,6 +126,7 @@ __device__ void cta_ig(const Inst &in, int64_t lo, int64_t hi, unsigned long lon
       if (live && k < m) v[u] = ld_table(in.aux + k);
       else if (live) nb++;
     }
+    load(i + U * kThreads);  // the next indices while the table's entries are on their way
 #pragma unroll
     for (int u = 0; u < U; u++)
       if (i + u * kThreads < hi) st_stream(in.out + i + u * kThreads, v[u]);
@@ -209,24 +234,29 @@ Inst make_inst(const bale_instance_t &x) {
   return d;
 }
 
+// Tasks are small so that the queue's end is short and its 304 blocks are
+// busy whatever mix of instances it has: of 256 histograms, 192 gathers and 64
+// graphs, up to 2^20 elements each, 2^17 updates, 2^15 requests and 2^13
+// nonzeros a task took 1550 us; 2^14, 2^13 and 2^12 take 1270; half of these
+// 1290.
 void plan_tasks(const bale_instance_t &x, int32_t k, const int64_t *host_off, std::vector<Planned> &plan) {
   if (x.n == 0) return;
   const int cls = size_class(x.kind == BALE_KIND_TRIANGLES ? x.m : x.n);
   if (x.kind == BALE_KIND_HISTO) {
     if (x.m <= kSmemCounters) {
       // each task sees several updates per counter so the flush stays cheap
-      int64_t tile = tuned("batch.histo_tile", cls, int64_t(1) << 17);
+      int64_t tile = tuned("batch.histo_tile", cls, cls == 2 ? int64_t(1) << 17 : int64_t(1) << 14);
       tile = std::max<int64_t>(tile, 4 * x.m);
       for (int64_t lo = 0; lo < x.n; lo += tile)
         plan.push_back({{kHistoSmem, k, lo, std::min(x.n, lo + tile)},
                         static_cast<double>(std::min(tile, x.n - lo)) * 0.5 + static_cast<double>(x.m)});
     } else {
-      const int64_t tile = tuned("batch.histo_l2_tile", cls, int64_t(1) << 17);
+      const int64_t tile = tuned("batch.histo_l2_tile", cls, cls == 2 ? int64_t(1) << 17 : int64_t(1) << 14);
       for (int64_t lo = 0; lo < x.n; lo += tile)
         plan.push_back({{kHistoL2, k, lo, std::min(x.n, lo + tile)}, static_cast<double>(std::min(tile, x.n - lo))});
     }
   } else if (x.kind == BALE_KIND_IG) {
-    const int64_t tile = tuned("batch.ig_tile", cls, int64_t(1) << 17);
+    const int64_t tile = tuned("batch.ig_tile", cls, cls == 2 ? int64_t(1) << 17 : int64_t(1) << 13);
     for (int64_t lo = 0; lo < x.n; lo += tile)
       plan.push_back({{kIgDirect, k, lo, std::min(x.n, lo + tile)},
                       static_cast<double>(std::min(tile, x.n - lo)) * (x.m * 8 > (int64_t(96) << 20) ? 2.0 : 1.0)});
@@ -256,7 +286,7 @@ void plan_tasks(const bale_instance_t &x, int32_t k, const int64_t *host_off, st
         i++;
       }
     }
-    const int64_t lnnz = tuned("batch.tri_light_rows", cls, 1 << 15);  // nonzeros per light task
+    const int64_t lnnz = tuned("batch.tri_light_rows", cls, cls ? 1 << 15 : 1 << 12);  // nonzeros per light task
     int64_t lo = 0;
     while (lo < x.n) {
       int64_t hi = lo, acc = 0;

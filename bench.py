@@ -342,33 +342,28 @@ def run_histo(ctx) -> dict:
     reps = args.steps + args.warmup
     ok = bool(np.array_equal(counts.cpu().numpy(), reps * want)) and int(bad.item()) == 0
     n = HISTO_UPDATES
-    algo = 72 * n  # 8 B index + 32 B sector read + 32 B write-back per update
-    # the bound that binds here: the L2 reduction rate into the same 10^6
-    # counters, measured live (the update without its index stream)
+    # what an update cannot do without: its index once, every counter once each way
+    algo = 8 * n + 16 * HISTO_COUNTS
+    # beside it the rate of plain L2 reductions into the same 10^6 counters,
+    # measured live (the update without its index stream): what one
+    # red.global.add.u64 per update is bound by, and the buckets are not
     probe = torch.zeros(HISTO_COUNTS, dtype=torch.int64, device=dev)
     red_ms = time_device(lambda: bale.l2_red_rate(probe, n), args.steps, args.warmup, between)
     red_peak = n / (red_ms / 1e3) / 1e9
     del probe
-    achieved = n / (ms / 1e3) / 1e9
-    dram = ctx["traffic"].get("histo", {}).get("dram_bytes_per_step")
     out = {"metric": "GUP/s histogram (10^9 updates/s)",
            "value": round(job_rate(n, ms_max / 1e3, ctx["dist"].world) / 1e9, 4), "unit": "GUP/s",
            "ms_per_step": round(ms_max, 4), "parity_ok": ok,
-           # the 8 MB table is L2-resident, so the bound is the L2's rate of
-           # 64-bit reductions, not HBM: one red.global.add.u64 per update
-           "roofline": {"bound": "l2", "kernel": "histo_global_kernel (plain L2 reductions)",
-                        "achieved": round(achieved, 2), "peak": round(red_peak, 2), "unit": "G reductions/s",
-                        "frac": round(achieved / red_peak, 4),
-                        "peak_source": "measured live in this run: bale_l2_red_rate issues the same "
-                                       "red.global.add.u64 at hashed positions of the same 10^6 counters with no "
-                                       "index stream (10^7 reductions), CUDA events",
-                        "ncu_l2_throughput_pct": 70.6, "ncu_source": "profiles/histo_plain_l2_1e6_counters.md",
-                        "traffic": dram, "dram_gbs": round(dram / (ms / 1e3) / 1e9, 1) if dram else None,
-                        "hbm_model": {"algorithmic_bytes_per_step": algo,
-                                      "achieved_gbs": round(algo / (ms / 1e3) / 1e9, 1),
-                                      "note": "72 B/update (index + sector read + write-back) applies to tables "
-                                              "beyond L2; it reads above HBM peak here"}},
-           "clocks": clocks.summary(), "gpu_launches": args.steps,
+           "roofline": roofline(ctx, "histo", algo, ms / 1e3,
+                                "bucket_partition_kernel (indices to buckets in shared memory) + "
+                                "bucket_count_kernel (a bucket's counters in shared memory)",
+                                note="algorithmic bytes: 8 B per index, 16 B per counter; both kernels are bound by "
+                                     "shared-memory atomics and latency, not by HBM"),
+           "l2_reduction_rate": {"value": round(red_peak, 2), "unit": "G reductions/s",
+                                 "ratio": round(n / (ms / 1e3) / 1e9 / red_peak, 4),
+                                 "what": "bale_l2_red_rate: red.global.add.u64 at hashed positions of the same 10^6 "
+                                         "counters, no index stream"},
+           "clocks": clocks.summary(), "gpu_launches": 2 * args.steps,
            "config": {"workload": "histo: 10^7 uniform updates into 10^6 int64 counters",
                       "updates": n, "counters": HISTO_COUNTS,
                       "l2": "inputs fit in L2: a 256 MiB buffer is rewritten between steps"}}
@@ -422,7 +417,7 @@ def run_triangles(ctx) -> dict:
     records = int(live.sum())
     del rowid, pos, live
     # the dominant kernels alone: counting from a prepared graph (the wedge
-    # probe kernel and the dense-pair kernel); their algorithmic bytes are the
+    # kernels of the near and the far rows); their algorithmic bytes are the
     # push model's -- every probed prefix element read once as a u32 (the
     # dense pairs counted as the pushes they replace), the 8-byte prefix
     # records, and rows j read twice (set and clear) as u32
@@ -434,20 +429,20 @@ def run_triangles(ctx) -> dict:
     out = {"metric": "edges/s triangle counting (nnz(L) per second)",
            "value": round(job_rate(nnz, ms_max / 1e3, ctx["dist"].world) / 1e9, 4), "unit": "Gedges/s",
            "ms_per_step": round(ms_max, 4), "triangles": per_step,
-           # the count kernel is bound by instruction issue (ncu: issue active
-           # ~69%, most probes served from L2), so its DRAM traffic (ncu,
-           # per launch) over the live kernel time is a fraction of HBM, and
-           # the push-model bytes (L2 + DRAM) are reported beside it
+           # the count kernels are bound by shared-memory lookups and by
+           # dependent loads, so their DRAM traffic (ncu, per launch) over the
+           # live kernel time is a fraction of HBM, and the push-model bytes
+           # (L2 + DRAM) are reported beside it
            "roofline": tri_roofline(ctx, wedge_bytes, count_ms / 1e3, ms_max),
            "roofline_pull_model": {"algorithmic_bytes_per_step": 8 * (n + 1) + 8 * nnz + 8 * pulls,
                                    "achieved_gbs": round((8 * (n + 1) + 8 * nnz + 8 * pulls) / ms_max * 1e-6, 1),
                                    "note": "the AGI loop's pull model (8 B per row-j element scanned); the "
                                            "wedge kernels probe 4x fewer elements, so this reads above 1"},
            "count_kernel_ms": round(count_ms, 4),
-           # per call: the path choice, the wedge scan, row bitmaps, hub scan, 3
-           # offset kernels, fill, probes, dense pairs, and the 4 hybrid kernels
+           # per call: the path choice, rows, scan, hubs, 3 offset kernels, fill,
+           # near rows with the dense pairs, far rows, and the 5 hybrid kernels
            # that return at once when the wedges are chosen
-           "clocks": clocks.summary(), "gpu_launches": 14 * args.steps,
+           "clocks": clocks.summary(), "gpu_launches": 15 * args.steps,
            "config": {"workload": "triangles: R-MAT scale 22, edge factor 16, (0.57,0.19,0.19,0.05), "
                                   "symmetrised, deduplicated, degree-ordered strictly lower L",
                       "n": n, "nnz": nnz, "pulls": pulls, "pushes": pushes, "generate_s": round(gen_s, 2),
@@ -524,23 +519,24 @@ def run_graph(ctx) -> dict:
     nnz = col.numel()
     offs_h, col_h = off.cpu().numpy(), col.cpu().numpy()
     maxdeg = int((np.diff(offs_h) + np.bincount(col_h, minlength=1 << S)).max())
-    p_edges, p_vert, p_lower = (2 * S + 1 + 7) // 8, (S + maxdeg.bit_length() + 7) // 8, (2 * S + 7) // 8
-    # the dominant work: three LSD radix sorts, each reading its 8-byte keys
-    # once for the digit counts of all passes, then every 8-bit pass reading
-    # and writing each key once
-    algo = 16 * (p_edges * m + p_vert * (1 << S) + p_lower * nnz) + 8 * (m + (1 << S) + nnz)
-    # edge keys, per sort the digit counts + starts + one kernel per pass,
-    # dedup (flag, 3 scan kernels, compact), max, vertex keys, labels, lower keys, CSR
-    launches = 1 + (2 + p_edges) + 1 + 3 + 1 + 1 + 1 + (2 + p_vert) + 1 + 1 + (2 + p_lower) + 2
+    p_vert, p_lower = (maxdeg.bit_length() + 7) // 8, (2 * S + 7) // 8
+    # the distinct edges: every key read twice (bucket sizes, partition),
+    # written to its bucket and read from it; two LSD radix sorts, each reading
+    # its 8-byte keys once for the digit counts of all passes, then every 8-bit
+    # pass reading and writing each key once
+    algo = 32 * m + 16 * (p_vert * (1 << S) + p_lower * nnz) + 8 * ((1 << S) + nnz)
+    # edge keys, distinct edges (4 kernels), degrees (2), max, vertex keys, per
+    # sort the digit counts + starts + one kernel per pass, labels, lower keys, CSR
+    launches = 1 + 4 + 2 + 1 + 1 + (2 + p_vert) + 1 + 1 + (2 + p_lower) + 2
     out = {"metric": "G input edges/s building the degree-ordered lower CSR (R-MAT scale 22) on the device",
            "value": round(job_rate(m, ms_max / 1e3, ctx["dist"].world) / 1e9, 4), "unit": "G edges/s",
            "ms_per_step": round(ms_max, 3), "nnz": nnz,
            "roofline": roofline(ctx, "graph", algo, ms / 1e3,
-                                "the build's radix sorts (one digit count per sort, one look-back scatter "
-                                "per 8-bit pass) and graph steps",
-                                note="algorithmic bytes: 16 B per key per 8-bit pass plus 8 B per key per sort "
-                                     "over the m edge keys (45 bits), the 2^22 vertex keys and the nnz lower keys "
-                                     "(44 bits); the generation, dedup and CSR steps are not counted"),
+                                "the build's distinct edges by hashed buckets and radix sorts (one digit count "
+                                "per sort, one look-back scatter per 8-bit pass)",
+                                note="algorithmic bytes: 32 B per edge key for the distinct edges, 16 B per key per "
+                                     "8-bit pass plus 8 B per key per sort over the 2^22 vertex keys and the nnz "
+                                     "lower keys (44 bits); the generation, degree and CSR steps are not counted"),
            "clocks": clocks.summary(), "gpu_launches": launches * args.steps,
            "config": {"workload": "R-MAT scale 22, edge factor 16, (0.57,0.19,0.19,0.05): 67,108,864 generated "
                                   "edges -> symmetrised, deduplicated, degree-ordered strictly lower CSR",
@@ -954,18 +950,19 @@ def run_serve(ctx) -> dict:
 
 
 def tri_roofline(ctx, push_bytes: int, count_s: float, step_ms: float) -> dict:
-    """The wedge count kernel's roofline: bound by instruction issue; DRAM
-    bytes per launch from the committed ncu capture over the live kernel
+    """The wedge count kernels' roofline: bound by shared-memory lookups (near
+    rows) and dependent loads (far rows); DRAM bytes per launch from the committed ncu capture over the live kernel
     time, against the measured HBM peak; the push-model bytes beside it."""
     tr = ctx["traffic"].get("triangles", {})
     dram = tr.get("dram_bytes_per_step")
     achieved = dram / count_s / 1e9 if dram else None
-    return {"bound": "issue", "kernel": "wedge_count_kernel (one warp per row j: bitmap / staged search over the "
-                                        "incoming prefixes) + wedge_dense_kernel (bitmap AND of the dense pairs)",
+    return {"bound": "shared memory", "kernel": "wedge_near_kernel (bitmap lookups of the prefixes of rows below "
+                                                "2^15, bitmap AND of the dense pairs) + wedge_far_kernel (the rows "
+                                                "from there on)",
             "achieved": round(achieved, 1) if achieved else None, "peak": ctx["peak"], "peak_source": ctx["peak_src"],
             "unit": "GB/s", "frac": round(achieved / ctx["peak"], 4) if achieved else None, "traffic": dram,
             "what": "DRAM bytes of one count (both kernels, ncu) over their live time: their share of HBM",
-            "issue_active_ncu": tr.get("issue_active"), "ncu_source": tr.get("summary"),
+            "shared_pipe_active_ncu": tr.get("shared_pipe_active"), "ncu_source": tr.get("summary"),
             "count_kernel_ms": round(count_s * 1e3, 4),
             "push_model": {"bytes_per_launch": push_bytes, "achieved_gbs": round(push_bytes / count_s / 1e9, 1),
                            "note": "4 B per probed prefix element (exstack pushes, "

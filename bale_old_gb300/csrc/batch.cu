@@ -372,9 +372,11 @@ void destroy(bale_batch *b) {
 namespace q {
 
 // Would this instance use the bucketed or region-partitioned kernels on its
-// own?  The planner gives it a workspace for them.
-static bool bucketed(const bale_instance_t &x) {
-  return x.kind == BALE_KIND_HISTO && histo_mode_for(x.n, x.m, x.in, false) == 4;
+// own?  The planner gives it a workspace for them; with own_ws, which is the
+// entry points' rule, already for the histograms of some 2^23 updates (the
+// uneven mix of 512 instances: 37.4 -> 34.9 ms).
+static bool bucketed(const bale_instance_t &x, bool own_ws) {
+  return x.kind == BALE_KIND_HISTO && histo_mode_for(x.n, x.m, x.in, own_ws) == 4;
 }
 
 bool partition_worthy(const bale_instance_t &x) {
@@ -392,10 +394,10 @@ bool goes_standalone(const bale_instance_t &x) {
   return x.n >= knob_or("batch.standalone_min", int64_t(1) << 23);
 }
 
-size_t standalone_ws(const bale_instance_t &x) {
+size_t standalone_ws(const bale_instance_t &x, bool own_ws) {
   size_t need = 0;
   if (x.kind == BALE_KIND_IG && partition_worthy(x)) need = ig_part_workspace_bytes(x.n, x.m);
-  else if (bucketed(x)) need = bucket_workspace_bytes(x.n, x.m);
+  else if (bucketed(x, own_ws)) need = bucket_workspace_bytes(x.n, x.m);
   else if (x.kind == BALE_KIND_HISTO && partition_worthy(x)) need = histo_part_workspace_bytes(x.n, x.m);
   else if (x.kind == BALE_KIND_TRIANGLES)
     need = tri_wedge_supported(x.n, x.m) ? tri_wedge_workspace_bytes(x.n, x.m) : tri_hybrid_workspace_bytes(x.n, x.m);
@@ -408,13 +410,13 @@ double standalone_cost(const bale_instance_t &x) {
 }
 
 int launch_standalone(const bale_instance_t &x, unsigned long long *bad, void *ws, unsigned long long *words,
-                      cudaStream_t st) {
+                      cudaStream_t st, bool own_ws) {
   if (x.kind == BALE_KIND_IG) {
     if (partition_worthy(x)) return launch_ig_partitioned(x.out, x.in, x.n, x.aux, x.m, x.shift, bad, ws, words, st);
     return launch_ig(x.out, x.in, x.n, x.aux, x.m, x.shift, bad, st, false);
   }
   if (x.kind == BALE_KIND_HISTO) {
-    if (bucketed(x)) return launch_histo_bucket(x.out, x.m, x.in, x.n, x.shift, bad, ws, st);
+    if (bucketed(x, own_ws)) return launch_histo_bucket(x.out, x.m, x.in, x.n, x.shift, bad, ws, st);
     if (partition_worthy(x)) return launch_histo_partitioned(x.out, x.m, x.in, x.n, x.shift, bad, ws, words, st);
     return launch_histo(x.out, x.m, x.in, x.n, x.shift, bad, st, false);
   }
@@ -479,16 +481,12 @@ bale_batch_t *bale_batch_create(const bale_instance_t *inst, int64_t count) {
 
   // ---- plan: standalone instances, then the work queue ----
   std::vector<Planned> plan;
-  std::vector<size_t> ws_off;
-  size_t ws_total = 256;
   std::vector<int64_t> host_off;
   for (int64_t k = 0; k < count; k++) {
     const bale_instance_t &x = inst[k];
     if (x.n == 0) continue;
     if (goes_standalone(x)) {
       b->standalone.push_back(k);
-      ws_off.push_back(ws_total);
-      ws_total += standalone_ws(x);
       continue;
     }
     if (x.kind == BALE_KIND_TRIANGLES) {
@@ -514,7 +512,25 @@ bale_batch_t *bale_batch_create(const bale_instance_t *inst, int64_t count) {
   BATCH_CUDA(cudaMalloc(&b->d_tasks, sizeof(Task) * std::max<size_t>(1, tasks.size())));
   BATCH_CUDA(cudaMalloc(&b->d_words, sizeof(unsigned long long) * nw));
   BATCH_CUDA(cudaMalloc(&b->d_bad, sizeof(unsigned long long) * std::max<int64_t>(1, count)));
-  if (!b->standalone.empty()) BATCH_CUDA(cudaMalloc(&b->d_ws, ws_total));
+  // the standalone instances' workspaces; without the entry points' rule for
+  // histograms where that many bytes cannot be had
+  std::vector<size_t> ws_off(b->standalone.size());
+  bool own_ws = true;
+  for (;; own_ws = false) {
+    size_t ws_total = 256;
+    for (size_t s = 0; s < ws_off.size(); s++) {
+      ws_off[s] = ws_total;
+      ws_total += standalone_ws(inst[b->standalone[s]], own_ws);
+    }
+    if (b->standalone.empty()) break;
+    if (!own_ws) {
+      BATCH_CUDA(cudaMalloc(&b->d_ws, ws_total));
+      break;
+    }
+    if (cudaMalloc(&b->d_ws, ws_total) == cudaSuccess) break;
+    cudaGetLastError();
+    b->d_ws = nullptr;
+  }
   if (!di.empty()) BATCH_CUDA(cudaMemcpy(b->d_inst, di.data(), sizeof(Inst) * di.size(), cudaMemcpyHostToDevice));
   if (!tasks.empty())
     BATCH_CUDA(cudaMemcpy(b->d_tasks, tasks.data(), sizeof(Task) * tasks.size(), cudaMemcpyHostToDevice));
@@ -580,7 +596,8 @@ bale_batch_t *bale_batch_create(const bale_instance_t *inst, int64_t count) {
     for (size_t s = 0; s < b->standalone.size() && cap_ok; s++) {
       const int64_t k = b->standalone[s];
       void *ws = static_cast<char *>(b->d_ws) + ws_off[s];
-      cap_ok &= launch_standalone(inst[k], b->d_bad + k, ws, b->d_words + 2 + 4 * s, b->s_side[lane[s]]) == BALE_OK;
+      cap_ok &= launch_standalone(inst[k], b->d_bad + k, ws, b->d_words + 2 + 4 * s, b->s_side[lane[s]],
+                                  own_ws) == BALE_OK;
     }
     for (int64_t l = 0; l < nside; l++) cap_ok &= cudaEventRecord(b->ev_join[l], b->s_side[l]) == cudaSuccess;
   }

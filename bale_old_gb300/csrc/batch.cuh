@@ -53,13 +53,14 @@ int launch_queue(const Task *d_tasks, int64_t ntasks, const Inst *d_inst, unsign
 // Large instances run as their own specialised kernels instead of queue
 // tasks: the rule (batch.standalone* knobs and the partition thresholds),
 // their workspace, a relative cost for stream balancing, and the launch
-// (words: 4 zero-initialised device words of cursors).
+// (words: 4 zero-initialised device words of cursors).  own_ws: the workspace
+// and the launch follow the entry points' rule for histograms; the same for both.
 bool partition_worthy(const bale_instance_t &x);
 bool goes_standalone(const bale_instance_t &x);
-size_t standalone_ws(const bale_instance_t &x);
+size_t standalone_ws(const bale_instance_t &x, bool own_ws = false);
 double standalone_cost(const bale_instance_t &x);
 int launch_standalone(const bale_instance_t &x, unsigned long long *bad, void *ws, unsigned long long *words,
-                      cudaStream_t st);
+                      cudaStream_t st, bool own_ws = false);
 
 }  // namespace q
 }  // namespace bale

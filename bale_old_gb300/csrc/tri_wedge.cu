@@ -23,7 +23,8 @@
 //      against 72 on average, and a graph of 2^14 rows gave 32 blocks work
 //      (R-MAT scale 22: fill 1515 -> 1077 us; 2^14 rows, 2^18 edges: fill
 //      77 -> 21 us, scan 41 -> 21);
-//   2. exclusive scan of the counts -> in_off;
+//   2. exclusive scan of the counts -> in_off, and the lists of the rows that
+//      are counted in parts;
 //   3. fill: in_rec[in_off[j] + t] = the prefix row_i[0,p): for near rows j
 //      (below 2^15) where its 16-bit copy starts and p, for the others i and p;
 //   4. count: one warp per j.  Row j's low columns (below 2^15 - 1) become a
@@ -37,8 +38,8 @@
 //      The prefixes are read from a copy of the rows in 16 bits, each row on
 //      a 16-byte boundary and padded so that whole vectors are probed without
 //      a test of where they end: 8 elements and 75 instructions per vector and
-//      lane instead of 4 and 108, half the bytes.  Warps claim equal shares of
-//      the records, not rows: a hub's 54 K prefixes took one warp 2.3 ms.
+//      lane instead of 4 and 108, half the bytes.  Rows with many records are
+//      claimed in parts: a hub's 54 K prefixes took one warp 2.3 ms.
 //      R-MAT scale 22, without the dense pairs of step 5:
 //      3980 us with 32-bit rows, a 2^16-bit bitmap per warp (24 warps an SM)
 //      and a claim per row; 2806 with 16-bit rows; 1850 as it is, near (40
@@ -47,9 +48,9 @@
 //      row j's high columns took 1163.
 //   5. dense pairs: a pair (i,j) whose prefix is long against the ceil(j/32)
 //      words of a bitmap of [0,j) (dense_pair below), for j below 2^14, gets no
-//      record in steps 1-3; step 1 also builds the column bitmaps of the rows
-//      below 2^14 and lists the rows i that have such pairs; warps claim these
-//      one by one, AND row i's bits with row j's and count them.
+//      record in steps 1-3; beside step 2 the column bitmaps of the rows below
+//      2^14 are built and the rows i that have such pairs listed; warps claim
+//      these one by one, AND row i's bits with row j's and count them.
 // Steps 1-3 and the bitmaps depend only on the matrix (a resident graph does
 // them once).  A malformed row raises *bad in step 1 and the later steps then
 // return at once; every index stays inside its array either way.  The work
@@ -129,7 +130,7 @@ enum {
 // column bitmap (j < hubs) and its prefix row_i[0,p) is longer than 3/8 of the
 // bitmap's ceil(j/32) words plus the margin ov: then one AND and popcount
 // per word of [0,j) costs less than p probes.  Dense pairs get no record;
-// wedge_dense_kernel counts them.  At R-MAT scale 22 a margin of 16 takes
+// dense_rows counts them.  At R-MAT scale 22 a margin of 16 takes
 // 4580 us a call with 3/8 of the words, 4640 with half, 4570 with a quarter,
 // about 4850 with all of them and a margin of 32.
 __device__ __forceinline__ bool dense_pair(uint32_t j, uint32_t p, int64_t ov, uint32_t hubs) {

@@ -1009,6 +1009,8 @@ __global__ void __launch_bounds__(kWarpThreads, kNearBlocksPerSm)
                       unsigned long long *__restrict__ count, unsigned long long *__restrict__ work,
                       unsigned long long *__restrict__ cursor, const unsigned *__restrict__ run_if) {
   if (tri::skipped(run_if, 1u)) return;
+  // the far kernel, which does not need this one's results, may begin
+  asm volatile("griddepcontrol.launch_dependents;");
   extern __shared__ __align__(16) uint32_t wsm[];
   if (words[kWBad]) return;
   const unsigned lane = lane_id();
@@ -1198,6 +1200,8 @@ __global__ void __launch_bounds__(kWarpThreads, kFarBlocksPerSm)
     }
   }
   flush(cnt, wk, count, work);
+  // the near kernel, beside which this one ran, is complete when this one is
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 bool g_far_attr[2][64];
@@ -1255,7 +1259,11 @@ int tri_wedge_prepare(const int64_t *offset, const int64_t *nonzero, int64_t num
     BALE_CUDA_OK(cudaGetLastError());
   }
   uint32_t *next = reinterpret_cast<uint32_t *>(p + l.next);
-  const uint32_t stage_max = static_cast<uint32_t>(std::min<int64_t>(knob_or("tri.wedge_stage_max", 64), kStageMax));
+  // far rows of more columns are long ones; below 2^16 rows there are enough
+  // warps to give each row of a dense matrix one (Erdos-Renyi, 60 K rows of 24
+  // columns: 108 us with 64, 78 with 16; sparser and larger ones lose by it)
+  const int64_t stage = knob_or("tri.wedge_stage_max", numrows < 65536 && nnz >= 16 * numrows ? 16 : 64);
+  const uint32_t stage_max = static_cast<uint32_t>(std::min<int64_t>(stage, kStageMax));
   wedge_offsets_kernel<<<static_cast<unsigned>(nb), kPsumThreads, 0, stream>>>(
       in_cnt, numrows, nb > kOwnPrefix ? bsum : nullptr, in_off, next, offset, reinterpret_cast<uint2 *>(p + l.nears),
       reinterpret_cast<uint2 *>(p + l.longs), stage_max, words, run_if);
@@ -1304,15 +1312,27 @@ int tri_wedge_run(const int64_t *offset, const void *ws, int64_t numrows, int64_
                                         static_cast<int>(kFarWords * sizeof(uint32_t) * kWarpWarps)));
       g_far_attr[wide][dev] = true;
     }
-    // windows of 32 rows; of fewer when there is not one for each of the GPU's
-    // warps (Erdos-Renyi, 50 K rows of 10: 113 us with 32 rows, 52 with 4)
+    // windows of 32 rows; of fewer when there are not three for each of the
+    // GPU's warps (Erdos-Renyi, 50 K rows of 10: 113 us with 32 rows, 52 with 4;
+    // 150 K of 24: 296 with 25, 240 with 8; R-MAT 2^18: 141 with 32, 120 with 16)
     const int64_t warps = static_cast<int64_t>(sms) * kFarBlocksPerSm * kWarpWarps, rows = numrows - near;
     const uint32_t window = static_cast<uint32_t>(
-        std::max<int64_t>(kWindowMin, std::min<int64_t>(32, (rows + warps - 1) / warps)));
-    far_kernel<<<blocks_for((rows + window - 1) / window + nnz / kPart, kFarBlocksPerSm), kWarpThreads,
-                 kFarWords * sizeof(uint32_t) * kWarpWarps, stream>>>(
-        offset, col32, rows16, l.nvec16, in_off, in_rec, numrows, window, nvec_all,
-        reinterpret_cast<const uint2 *>(p + l.longs), words, count, work, cursor + 1, run_if);
+        std::max<int64_t>(kWindowMin, std::min<int64_t>(32, (rows + 3 * warps - 1) / (3 * warps))));
+    // beside the near kernel, with whose work this one has nothing to do but
+    // the tallies (R-MAT 2^16 prepared 65 -> 58 us, 2^18 130 -> 120)
+    cudaLaunchAttribute beside{};
+    beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    beside.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks_for((rows + window - 1) / window + nnz / kPart, kFarBlocksPerSm));
+    cfg.blockDim = dim3(kWarpThreads);
+    cfg.dynamicSmemBytes = kFarWords * sizeof(uint32_t) * kWarpWarps;
+    cfg.stream = stream;
+    cfg.attrs = &beside;
+    cfg.numAttrs = 1;
+    BALE_CUDA_OK(cudaLaunchKernelEx(&cfg, far_kernel, offset, col32, rows16, static_cast<uint64_t>(l.nvec16), in_off,
+                                    in_rec, numrows, window, nvec_all, reinterpret_cast<const uint2 *>(p + l.longs),
+                                    words, count, work, cursor + 1, run_if));
     BALE_CUDA_OK(cudaGetLastError());
   }
   return BALE_OK;

@@ -69,7 +69,9 @@ Knob g_knobs[] = {
     {"sort.lookback_spins", -1},  // reads without progress before a sort pass's look-back gives up (2^22)
     {"sort.test_withhold", -1},   // 1: tile 0 of each sort pass publishes nothing (tests the bounded wait)
     {"tri.mode", -1},           // 0 warp-per-row merge, 1 bitmap/search hybrid, 2 wedge probes; -1 per graph
-    {"tri.wedge_stage_max", -1}, // wedge mode: rows from 2^15 on with at most this many columns are binary-searched (64)
+    // wedge mode: rows from 2^15 on with at most this many columns are binary-searched
+    // (64; 16 in dense matrices below 2^16 rows)
+    {"tri.wedge_stage_max", -1},
     {"tri.wedge_pull_pct", -1},     // default mode: wedges when pulls >= this % of pushes (192)
     {"tri.wedge_push_per_nnz", -1}, // ... or when pushes >= this many per nonzero (no such clause)
     {"tri.choose_min_nnz", -1},     // the per-graph choice from this many nonzeros; wedges below (2^23)
